@@ -21,6 +21,7 @@
 #include "engine_internal.h"
 #include "negf_gpu.h"
 #include "rgf_device.cuh"
+#include "sweep_kernels.h"
 
 using namespace negf;
 
@@ -30,127 +31,8 @@ constexpr double PI = 3.141592653589793;           // global.f90:28
 constexpr double HARTREE = 27.211386245988;        // global.f90:24
 constexpr double K_B = 8.617333262e-5 / HARTREE;   // global.f90:26
 
-struct RgfJob {
-    double e_re, e_im;  // complex energy of the solve, E + i*eta already added
-    double e_t;         // real energy of the transmission weights
-    int ik;             // k-point
-    int pad;
-    // WANT_A only: slice k of the output is cd * G_kk + ca * G_k,s Gamma_s G_k,s^H
-    // (s = the injecting lead's end slice, Gamma_s its open-channel widths)
-    double cd_re, cd_im, ca_re, ca_im;
-};
 
 // ------------------------------------------------------------------ kernels
-// One F-mode sweep and the transmission trace for the job (E = e + i*eta,
-// k-point ik) of problem g, in the workspace A0 (four ld x N blocks).  The
-// basis must already be in s.nx / s.ny.  Returns tau in *tau (thread 0) and
-// the LAPACK-style info.
-template <int NB, int RPT>
-__device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, double2 *A0, double *tau) {
-    const int N = g.N, ld = g.ld, Nz = g.Nz;
-    double2 *A1 = A0 + (size_t)ld * N;
-    double2 *P0 = A1 + (size_t)ld * N;
-    double2 *P1 = P0 + (size_t)ld * N;
-    const double2 E = make_double2(e, g.eta);
-    job_vectors(g, s, E, e, ik);
-    __syncthreads();
-    open_rows(N, s);
-    __syncthreads();
-    const int nr = *s.nrows;
-    double2 *cur = A0, *oth = A1, *P = P0, *Pn = P1;
-    // generator_r(N_z-1) = inv(D_Nz)          math_kernel.f90:82
-    form_block(cur, g, s, Nz - 1, E, ik, nullptr, nullptr);
-    __syncthreads();
-    int info = gj_invert<NB, RPT>(cur, N, ld, s);
-    unpermute_rows(P, ld, cur, ld, N, nr, s);
-    __syncthreads();
-    // generator_r(m) = inv(D_{m+1} - generator_r(m+1)), with the rows of the
-    // running product P = gR(Nz-1) ... gR(m) of the first-column chain
-    // G_{Nz,1} = (-1)^(Nz-1) gR(Nz-1) ... gR(1) G_11 (math_kernel.f90:83-90,120-128)
-    // that the trace reads
-    for (int m = Nz - 3; m >= 0; --m) {
-        form_block(oth, g, s, m + 1, E, ik, cur, nullptr);
-        __syncthreads();
-        const int r = gj_invert<NB, RPT>(oth, N, ld, s);
-        if (r && !info) info = r;
-        GemmArgs ga{Pn, ld, P, ld, s.iprow, oth, ld, s.iprow, nr, N, N, nullptr};
-        cta_gemm(ga, s, GEMM_STORE, g.delta);
-        __syncthreads();
-        double2 *t = cur; cur = oth; oth = t;
-        t = P; P = Pn; Pn = t;
-    }
-    // G_11 = inv(D_1 - generator_r(1))          math_kernel.f90:113-118
-    form_block(oth, g, s, 0, E, ik, cur, nullptr);
-    __syncthreads();
-    const int r = gj_invert<NB, RPT>(oth, N, ld, s);
-    if (r && !info) info = r;
-    // tau = sum_ij gamma_L,i gamma_R,j |2 dz^2 G_{Nz,1}(i,j)|^2   grid.f90:362-383
-    GemmArgs ga{nullptr, 0, P, ld, s.iprow, oth, ld, s.iprow, nr, N, N, s.rows};
-    double t = cta_gemm(ga, s, GEMM_TAU, g.delta);
-    t = block_sum(t, s);
-    *tau = t;
-    return info;
-}
-
-template <int NB, int RPT, int MINB>
-__global__ void __launch_bounds__(NT, MINB)
-    k_transmission(Geo g, const double *__restrict__ energies, int nE, int njobs, double2 *ws,
-                   size_t wstride, double *tau_jobs, int *info_jobs) {
-    extern __shared__ __align__(256) unsigned char smem[];
-    Smem s = carve<NB>(smem, g.N);
-    for (int i = threadIdx.x; i < g.N; i += NT) { s.nx[i] = g.nx[i]; s.ny[i] = g.ny[i]; }
-    __syncthreads();
-    double2 *A0 = ws + (size_t)blockIdx.x * wstride;
-    for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
-        // job -> (energy, k-point), energy fastest: negf.f90:131-133
-        const int ie = job % nE, ik = job / nE;
-        double t = 0.0;
-        const int info = transmission_job<NB, RPT>(g, s, energies[ie], ik, A0, &t);
-        if (threadIdx.x == 0) {
-            tau_jobs[job] = t;
-            if (info_jobs) info_jobs[job] = info;
-        }
-        __syncthreads();
-    }
-}
-
-// One (problem, energy, k-point) job of a batch over several problems.
-struct BatchJob {
-    int prob, ie, ik, pad;
-};
-
-// Several problems (each its own basis, V table, slices and k-points) in one
-// persistent launch: CTAs take jobs from a counter in the given order
-// (largest first), so long and short sweeps balance across the SMs.
-template <int NB, int RPT, int MINB>
-__global__ void __launch_bounds__(NT, MINB)
-    k_transmission_batch(const Geo *__restrict__ geos, const BatchJob *__restrict__ jobs, int njobs,
-                         const double *__restrict__ energies, double2 *ws, size_t wstride, double *tau_jobs,
-                         int *info_jobs, int *counter) {
-    extern __shared__ __align__(256) unsigned char smem[];
-    __shared__ int next;
-    double2 *A0 = ws + (size_t)blockIdx.x * wstride;
-    for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(counter, 1);
-        __syncthreads();
-        const int q = next;
-        __syncthreads();
-        if (q >= njobs) break;
-        const BatchJob jb = jobs[q];
-        const Geo g = geos[jb.prob];
-        Smem s = carve<NB>(smem, g.N);
-        for (int i = threadIdx.x; i < g.N; i += NT) { s.nx[i] = g.nx[i]; s.ny[i] = g.ny[i]; }
-        __syncthreads();
-        double t = 0.0;
-        const int info = transmission_job<NB, RPT>(g, s, energies[jb.ie], jb.ik, A0, &t);
-        if (threadIdx.x == 0) {
-            tau_jobs[q] = t;
-            info_jobs[q] = info;
-        }
-        __syncthreads();
-    }
-}
-
 // tau(E) = sum_k w_k tau(E,k)   negf.f90:172
 __global__ void k_tau_reduce(const double *__restrict__ tau_jobs, const double *__restrict__ kw, int nE,
                              int nk, double *__restrict__ tau) {
@@ -159,185 +41,6 @@ __global__ void k_tau_reduce(const double *__restrict__ tau_jobs, const double *
     double t = 0.0;
     for (int ik = 0; ik < nk; ++ik) t += tau_jobs[(size_t)ik * nE + ie] * kw[ik];
     tau[ie] = t;
-}
-
-enum { WANT_D = 1, WANT_F = 2, WANT_L = 4, WANT_A = 8, WANT_MIRROR = 16 };
-
-// One job per CTA.  slab (Nz blocks, leading dimension ld) first receives
-// the generator_r blocks; with WANT_D it ends up holding G_kk in block k.
-// out_first / out_last (leading dimension N) receive G_k1 / G_kNz.
-// WANT_A (with WANT_D): block k becomes cd * G_kk + ca * A_k, where
-// A_k = G_k1 Gamma_L G_k1^H is the spectral function injected by the left
-// lead, restricted to its open channels: Y_1 = G_11(:, open) sqrt(gamma_L),
-// Y_k = -gR(k-1) Y_{k-1}, A_k = Y_k Y_k^H (8 n_open N^2 flop per product).
-// WANT_MIRROR runs the same recursions with the slices numbered from the
-// right end (left-connected generators; the injecting lead is the right
-// one), writing every block at its own slice index.  Workspace: 6 blocks.
-template <int NB, int RPT, int MINB>
-__global__ void __launch_bounds__(NT, MINB)
-    k_rgf_slab(Geo g, const RgfJob *__restrict__ jobs, int njobs, const double2 *__restrict__ Dexp,
-               double2 *ws, size_t wstride, double2 *slabs, size_t sstride, int want,
-               double2 *out_first, double2 *out_last, int *info_jobs) {
-    extern __shared__ __align__(256) unsigned char smem[];
-    Smem s = carve<NB>(smem, g.N);
-    const int N = g.N, ld = g.ld, Nz = g.Nz;
-    const size_t NB2 = (size_t)ld * N;  // one workspace block
-    const size_t NN = (size_t)N * N;    // one output block
-    for (int i = threadIdx.x; i < N; i += NT) { s.nx[i] = g.nx[i]; s.ny[i] = g.ny[i]; }
-    __syncthreads();
-    const int job = blockIdx.x;
-    if (job >= njobs) return;
-    double2 *A0 = ws + (size_t)blockIdx.x * wstride;
-    double2 *A1 = A0 + NB2, *T0 = A1 + NB2, *T1 = T0 + NB2, *T2 = T1 + NB2, *Zt = T2 + NB2;
-    double2 *slab = slabs + (size_t)blockIdx.x * sstride;
-    const bool mirror = (want & WANT_MIRROR) != 0;
-    // slice of step x, and the slab block that holds it
-    auto sl = [&](int x) { return mirror ? Nz - 1 - x : x; };
-    auto blk = [&](int x) { return slab + NB2 * sl(x); };
-    const RgfJob jb = jobs[job];
-    const double2 E = make_double2(jb.e_re, jb.e_im);
-    const int ik = jb.ik;
-    if (!Dexp) job_vectors(g, s, E, jb.e_t, ik);
-    __syncthreads();
-    int info = 0, r;
-    double2 *cur = A0, *oth = A1;
-
-    if (want & (WANT_D | WANT_F)) {
-        // generator_r, math_kernel.f90:81-91
-        form_block(cur, g, s, sl(Nz - 1), E, ik, nullptr, Dexp);
-        __syncthreads();
-        info = gj_invert<NB, RPT>(cur, N, ld, s);
-        unpermute(blk(Nz - 2), ld, cur, ld, N, s, 1.0);
-        __syncthreads();
-        for (int m = Nz - 3; m >= 0; --m) {
-            form_block(oth, g, s, sl(m + 1), E, ik, cur, Dexp);
-            __syncthreads();
-            r = gj_invert<NB, RPT>(oth, N, ld, s);
-            if (r && !info) info = r;
-            unpermute(blk(m), ld, oth, ld, N, s, 1.0);
-            __syncthreads();
-            double2 *t = cur; cur = oth; oth = t;
-        }
-        form_block(oth, g, s, sl(0), E, ik, cur, Dexp);
-        __syncthreads();
-        r = gj_invert<NB, RPT>(oth, N, ld, s);
-        if (r && !info) info = r;
-        unpermute(T0, ld, oth, ld, N, s, 1.0);  // T0 = G_11
-        __syncthreads();
-        if ((want & WANT_F) && out_first) {
-            // G_k1 = -gR(k-1) G_{k-1,1}, math_kernel.f90:112-129
-            for (int e = threadIdx.x; e < N * N; e += NT) {
-                const int i = e % N, j = e / N;
-                out_first[e] = T0[i + (size_t)ld * j];
-            }
-            __syncthreads();
-            for (int k = 1; k < Nz; ++k) {
-                GemmArgs ga{out_first + NN * k, N, slab + NB2 * (k - 1), ld, nullptr,
-                            out_first + NN * (k - 1), N, nullptr, N, N, N, nullptr};
-                cta_gemm(ga, s, GEMM_STORE_NEG, g.delta);
-                __syncthreads();
-            }
-        }
-        if (want & WANT_D) {
-            // G_kk = gR(k-1) (I + G_{k-1,k-1} gR(k-1)), math_kernel.f90:94-109.
-            // Block k-1 of the slab is replaced by G_{k-1,k-1} once gR(k-1)
-            // has been used for the last time.
-            const bool wa = (want & WANT_A) != 0;
-            const double2 cd = wa ? make_double2(jb.cd_re, jb.cd_im) : make_double2(1.0, 0.0);
-            const double2 ca = make_double2(jb.ca_re, jb.ca_im);
-            int nA = 0;
-            double2 *Ya = A0, *Yb = A1;  // A0, A1 are free once the sweep is done
-            if (wa && (ca.x != 0.0 || ca.y != 0.0)) {
-                const double *gam = mirror ? s.gR : s.gL;
-                open_cols(N, s, gam);
-                __syncthreads();
-                nA = *s.nrows;
-                for (int e = threadIdx.x; e < N * nA; e += NT) {
-                    const int i = e % N, c = e / N, j = s.rows[c];
-                    const double sg = sqrt(gam[j]);
-                    const double2 v = T0[i + (size_t)ld * j];
-                    Ya[e] = make_double2(v.x * sg, v.y * sg);
-                }
-                __syncthreads();
-            }
-            // block += ca * Y Y^H, through Zt = Y^H (nA x N)
-            auto add_spectral = [&](double2 *dst, const double2 *Y) {
-                for (int e = threadIdx.x; e < N * nA; e += NT) {
-                    const int i = e % N, c = e / N;
-                    Zt[c + (size_t)nA * i] = make_double2(Y[e].x, -Y[e].y);
-                }
-                __syncthreads();
-                GemmArgs ga{dst, ld, Y, N, nullptr, Zt, nA, nullptr, N, N, nA, nullptr, ca};
-                cta_gemm(ga, s, GEMM_ADD_SCALED, g.delta);
-                __syncthreads();
-            };
-            double2 *Gc = T0, *Gn = T2;
-            for (int k = 1; k < Nz; ++k) {
-                double2 *gRk = blk(k - 1);
-                if (nA) {
-                    GemmArgs gy{Yb, N, gRk, ld, nullptr, Ya, N, nullptr, N, nA, N, nullptr};
-                    cta_gemm(gy, s, GEMM_STORE_NEG, g.delta);
-                    __syncthreads();
-                }
-                GemmArgs g1{T1, ld, Gc, ld, nullptr, gRk, ld, nullptr, N, N, N, nullptr};
-                cta_gemm(g1, s, GEMM_STORE_ADD_EYE, g.delta);
-                __syncthreads();
-                GemmArgs g2{Gn, ld, gRk, ld, nullptr, T1, ld, nullptr, N, N, N, nullptr};
-                cta_gemm(g2, s, GEMM_STORE, g.delta);
-                __syncthreads();
-                for (int e = threadIdx.x; e < N * N; e += NT) {
-                    const int i = e % N, j = e / N;
-                    gRk[i + (size_t)ld * j] = zmul(cd, Gc[i + (size_t)ld * j]);
-                }
-                __syncthreads();
-                if (nA) {
-                    add_spectral(gRk, Ya);
-                    double2 *t = Ya; Ya = Yb; Yb = t;
-                }
-                double2 *t = Gc; Gc = Gn; Gn = t;
-            }
-            double2 *last = blk(Nz - 1);
-            for (int e = threadIdx.x; e < N * N; e += NT) {
-                const int i = e % N, j = e / N;
-                last[i + (size_t)ld * j] = zmul(cd, Gc[i + (size_t)ld * j]);
-            }
-            __syncthreads();
-            if (nA) add_spectral(last, Ya);
-        }
-    }
-    if ((want & WANT_L) && out_last) {
-        // generator_l and the last column, math_kernel.f90:132-162; the
-        // generator_l blocks reuse slab blocks 0..Nz-2 (D/F are done with it).
-        cur = A0; oth = A1;
-        form_block(cur, g, s, 0, E, ik, nullptr, Dexp);
-        __syncthreads();
-        r = gj_invert<NB, RPT>(cur, N, ld, s);
-        if (r && !info) info = r;
-        unpermute(slab, ld, cur, ld, N, s, 1.0);
-        __syncthreads();
-        for (int m = 1; m <= Nz - 2; ++m) {
-            form_block(oth, g, s, m, E, ik, cur, Dexp);
-            __syncthreads();
-            r = gj_invert<NB, RPT>(oth, N, ld, s);
-            if (r && !info) info = r;
-            unpermute(slab + NB2 * m, ld, oth, ld, N, s, 1.0);
-            __syncthreads();
-            double2 *t = cur; cur = oth; oth = t;
-        }
-        form_block(oth, g, s, Nz - 1, E, ik, cur, Dexp);
-        __syncthreads();
-        r = gj_invert<NB, RPT>(oth, N, ld, s);
-        if (r && !info) info = r;
-        unpermute(out_last + NN * (Nz - 1), N, oth, ld, N, s, 1.0);
-        __syncthreads();
-        for (int k = 1; k < Nz; ++k) {
-            GemmArgs ga{out_last + NN * (Nz - 1 - k), N, slab + NB2 * (Nz - 1 - k), ld, nullptr,
-                        out_last + NN * (Nz - k), N, nullptr, N, N, N, nullptr};
-            cta_gemm(ga, s, GEMM_STORE_NEG, g.delta);
-            __syncthreads();
-        }
-    }
-    if (threadIdx.x == 0 && info_jobs) info_jobs[job] = info;
 }
 
 // out[o](i,j,k) (+)= sum_{q<gsz} coef[o*gsz+q] * ((slab_{o*gsz+q}(i,j,k) * 2) * dz^2)
@@ -590,7 +293,6 @@ int ensure_jobs(negf_ctx *c, int nE, int njobs) {
 
 // Kernel variants by basis size: (panel width NB, rows per thread RPT,
 // CTAs per SM).  Up to 256 plane waves two CTAs share an SM.
-enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, V8x1 = 3, VNONE = 4 };
 Variant pick_variant(int N) {
     if (N <= NT) return V16x1;
     if (N <= 2 * NT) return V16x2;
@@ -610,36 +312,36 @@ Variant transmission_variant(int N) { return N <= NT ? V8x1 : pick_variant(N); }
 Variant ctx_variant(const negf_ctx *c) {
     return (c->variant >= 0 && variant_fits(c->variant, c->N)) ? (Variant)c->variant : transmission_variant(c->N);
 }
-size_t variant_smem(Variant v, int N) {
-    switch (v) {
-        case V16x1: return smem_bytes<16>(N);
-        case V16x2: return smem_bytes<16>(N);
-        case V8x4: return smem_bytes<8>(N);
-        case V8x1: return smem_bytes<8>(N);
-        default: return 0;
-    }
-}
-
-template <typename K>
-int prep_kernel(K kern, size_t smem, int *occ) {
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// Opts a kernel into its dynamic shared memory; *occ = its resident CTAs per SM.
+int prep_kernel(const void *fn, int threads, size_t smem, int *occ) {
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int o = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, NT, smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, smem));
     *occ = o > 0 ? o : 1;
     return 0;
 }
 
-// CTAs of the transmission kernel resident per SM for this N.
+// The one-problem form of k on njobs jobs.
+int launch_one(const SweepKernel &k, int grid, Geo g, const double *d_E, int nE, int njobs, double2 *ws, size_t wstride,
+               double *d_tau_jobs, int *d_info, cudaStream_t st) {
+    void *args[] = {&g, &d_E, &nE, &njobs, &ws, &wstride, &d_tau_jobs, &d_info};
+    CK(cudaLaunchKernel(k.one, dim3(grid), dim3(k.threads), args, k.smem, st));
+    return 0;
+}
+
+// The batch form of k.
+int launch_batch(const SweepKernel &k, int grid, const Geo *d_geo, const BatchJob *d_jobs, int njobs, const double *d_E,
+                 double2 *ws, size_t wstride, double *d_tj, int *d_info, int *d_counter, cudaStream_t st) {
+    void *args[] = {&d_geo, &d_jobs, &njobs, &d_E, &ws, &wstride, &d_tj, &d_info, &d_counter};
+    CK(cudaLaunchKernel(k.batch, dim3(grid), dim3(k.threads), args, k.smem, st));
+    return 0;
+}
+
+// CTAs of the slab kernel resident per SM for this N.
 int resident_ctas(int N) {
-    const Variant v = pick_variant(N);
-    const size_t smem = variant_smem(v, N);
+    const SlabKernel k = slab_kernel(pick_variant(N), N);
     int occ = 1;
-    switch (v) {
-        case V16x1: prep_kernel(k_transmission<16, 1, 2>, smem, &occ); break;
-        case V16x2: prep_kernel(k_transmission<16, 2, 1>, smem, &occ); break;
-        case V8x4: prep_kernel(k_transmission<8, 4, 1>, smem, &occ); break;
-        default: break;
-    }
+    if (k.fn) prep_kernel(k.fn, k.threads, k.smem, &occ);
     return occ;
 }
 
@@ -648,36 +350,13 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
     const int njobs = nE * c->nk;
     const Variant v = ctx_variant(c);
     if (v == VNONE) return NEGF_ERR_UNSUPPORTED;
-    const size_t smem = variant_smem(v, c->N);
-    int occ = 1, rc = 0;
-    switch (v) {
-        case V16x1: rc = prep_kernel(k_transmission<16, 1, 2>, smem, &occ); break;
-        case V16x2: rc = prep_kernel(k_transmission<16, 2, 1>, smem, &occ); break;
-        case V8x1: rc = prep_kernel(k_transmission<8, 1, 2>, smem, &occ); break;
-        default: rc = prep_kernel(k_transmission<8, 4, 1>, smem, &occ); break;
-    }
+    const SweepKernel k = sweep_kernel(v, c->N);
+    int occ = 1;
+    int rc = prep_kernel(k.one, k.threads, k.smem, &occ);
     if (rc) return rc;
     const int grid = std::min(njobs, c->num_sms * occ);
-    const size_t wstride = 4 * (size_t)c->ld * c->N;
-    rc = ensure_ws(c, sizeof(double2) * wstride * grid);
-    if (rc) return rc;
-    Geo g = make_geo(c);
-    double2 *ws = (double2 *)c->d_ws;
-    switch (v) {
-        case V16x1:
-            k_transmission<16, 1, 2><<<grid, NT, smem, st>>>(g, d_E, nE, njobs, ws, wstride, d_tau_jobs, d_info);
-            break;
-        case V16x2:
-            k_transmission<16, 2, 1><<<grid, NT, smem, st>>>(g, d_E, nE, njobs, ws, wstride, d_tau_jobs, d_info);
-            break;
-        case V8x1:
-            k_transmission<8, 1, 2><<<grid, NT, smem, st>>>(g, d_E, nE, njobs, ws, wstride, d_tau_jobs, d_info);
-            break;
-        default:
-            k_transmission<8, 4, 1><<<grid, NT, smem, st>>>(g, d_E, nE, njobs, ws, wstride, d_tau_jobs, d_info);
-            break;
-    }
-    CK(cudaGetLastError());
+    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * grid))) return rc;
+    if ((rc = launch_one(k, grid, make_geo(c), d_E, nE, njobs, (double2 *)c->d_ws, k.ws, d_tau_jobs, d_info, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(d_tau_jobs, c->d_kw, nE, c->nk, d_tau);
     CK(cudaGetLastError());
     return 0;
@@ -686,32 +365,17 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
 int slab_launch(negf_ctx *c, const Geo &g, const RgfJob *d_jobs, int njobs, const double2 *d_D,
                 double2 *d_slabs, size_t sstride, int want, double2 *d_first, double2 *d_last,
                 int *d_info, cudaStream_t st) {
-    const Variant v = pick_variant(g.N);
-    if (v == VNONE) return NEGF_ERR_UNSUPPORTED;
-    const size_t smem = variant_smem(v, g.N);
-    const size_t wstride = 6 * (size_t)g.ld * g.N;
+    const SlabKernel k = slab_kernel(pick_variant(g.N), g.N);
+    if (!k.fn) return NEGF_ERR_UNSUPPORTED;
+    size_t wstride = 6 * (size_t)g.ld * g.N;
     int rc = ensure_ws(c, sizeof(double2) * wstride * njobs);
     if (rc) return rc;
     double2 *ws = (double2 *)c->d_ws;
     int occ = 1;
-    switch (v) {
-        case V16x1:
-            if ((rc = prep_kernel(k_rgf_slab<16, 1, 2>, smem, &occ))) return rc;
-            k_rgf_slab<16, 1, 2><<<njobs, NT, smem, st>>>(g, d_jobs, njobs, d_D, ws, wstride, d_slabs, sstride,
-                                                           want, d_first, d_last, d_info);
-            break;
-        case V16x2:
-            if ((rc = prep_kernel(k_rgf_slab<16, 2, 1>, smem, &occ))) return rc;
-            k_rgf_slab<16, 2, 1><<<njobs, NT, smem, st>>>(g, d_jobs, njobs, d_D, ws, wstride, d_slabs, sstride,
-                                                           want, d_first, d_last, d_info);
-            break;
-        default:
-            if ((rc = prep_kernel(k_rgf_slab<8, 4, 1>, smem, &occ))) return rc;
-            k_rgf_slab<8, 4, 1><<<njobs, NT, smem, st>>>(g, d_jobs, njobs, d_D, ws, wstride, d_slabs, sstride,
-                                                          want, d_first, d_last, d_info);
-            break;
-    }
-    CK(cudaGetLastError());
+    if ((rc = prep_kernel(k.fn, k.threads, k.smem, &occ))) return rc;
+    Geo gg = g;
+    void *args[] = {&gg, &d_jobs, &njobs, &d_D, &ws, &wstride, &d_slabs, &sstride, &want, &d_first, &d_last, &d_info};
+    CK(cudaLaunchKernel(k.fn, dim3(njobs), dim3(k.threads), args, k.smem, st));
     return 0;
 }
 
@@ -1318,18 +982,12 @@ int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const
     if (var == VNONE) return NEGF_ERR_UNSUPPORTED;
     std::vector<BatchJob> jobs(njobs);
     for (int q = 0; q < njobs; ++q) jobs[q] = BatchJob{0, ie[q], ik[q], 0};
-    const size_t smem = variant_smem(var, c->N);
-    int occ = 1, rc = 0;
-    switch (var) {
-        case V16x1: rc = prep_kernel(k_transmission_batch<16, 1, 2>, smem, &occ); break;
-        case V8x1: rc = prep_kernel(k_transmission_batch<8, 1, 2>, smem, &occ); break;
-        case V16x2: rc = prep_kernel(k_transmission_batch<16, 2, 1>, smem, &occ); break;
-        default: rc = prep_kernel(k_transmission_batch<8, 4, 1>, smem, &occ); break;
-    }
+    const SweepKernel k = sweep_kernel(var, c->N);
+    int occ = 1;
+    int rc = prep_kernel(k.batch, k.threads, k.smem, &occ);
     if (rc) return rc;
     const int grid = std::min(njobs, c->num_sms * occ);
-    const size_t wstride = 4 * (size_t)c->ld * c->N;
-    if ((rc = ensure_ws(c, sizeof(double2) * wstride * grid))) return rc;
+    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * grid))) return rc;
     Geo g = make_geo(c);
     Geo *d_geo = nullptr;
     BatchJob *d_jobs = nullptr;
@@ -1346,22 +1004,8 @@ int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const
                 cudaMemsetAsync(d_counter, 0, sizeof(int), st) || cudaEventRecord(c->ev0, st)))
         rc = NEGF_ERR_CUDA;
     if (!rc) {
-        double2 *ws = (double2 *)c->d_ws;
-        switch (var) {
-            case V16x1:
-                k_transmission_batch<16, 1, 2><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                break;
-            case V16x2:
-                k_transmission_batch<16, 2, 1><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                break;
-            case V8x1:
-                k_transmission_batch<8, 1, 2><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                break;
-            default:
-                k_transmission_batch<8, 4, 1><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                break;
-        }
-        if (cudaGetLastError() || cudaEventRecord(c->ev1, st) ||
+        rc = launch_batch(k, grid, d_geo, d_jobs, njobs, d_E, (double2 *)c->d_ws, k.ws, d_tj, d_info, d_counter, st);
+        if (rc || cudaEventRecord(c->ev1, st) ||
             cudaMemcpyAsync(h_tau, d_tj, sizeof(double) * njobs, cudaMemcpyDeviceToHost, st) ||
             cudaMemcpyAsync(h_info, d_info, sizeof(int) * njobs, cudaMemcpyDeviceToHost, st) ||
             cudaStreamSynchronize(st) || cudaEventElapsedTime(ms, c->ev0, c->ev1))
@@ -1434,19 +1078,11 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         std::vector<BatchJob> sorted(jobs.size());
         for (size_t q = 0; q < order.size(); ++q) sorted[q] = jobs[order[q]];
         const int njobs = (int)sorted.size();
-        const Variant var = (Variant)v;
-        const size_t smem = variant_smem(var, nmax);
+        const SweepKernel k = sweep_kernel((Variant)v, nmax);
         int occ = 1;
-        switch (var) {
-            case V16x1: rc = prep_kernel(k_transmission_batch<16, 1, 2>, smem, &occ); break;
-            case V8x1: rc = prep_kernel(k_transmission_batch<8, 1, 2>, smem, &occ); break;
-            case V16x2: rc = prep_kernel(k_transmission_batch<16, 2, 1>, smem, &occ); break;
-            default: rc = prep_kernel(k_transmission_batch<8, 4, 1>, smem, &occ); break;
-        }
-        if (rc) break;
+        if ((rc = prep_kernel(k.batch, k.threads, k.smem, &occ))) break;
         const int grid = std::min(njobs, c0->num_sms * occ);
-        const size_t wstride = 4 * (size_t)round_up(nmax, 8) * nmax;
-        if ((rc = ensure_ws(c0, sizeof(double2) * wstride * grid))) break;
+        if ((rc = ensure_ws(c0, sizeof(double2) * k.ws * grid))) break;
         Geo *d_geo = nullptr;
         BatchJob *d_jobs = nullptr;
         double *d_tj = nullptr;
@@ -1469,22 +1105,8 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
                 rc = NEGF_ERR_CUDA;
         }
         if (!rc) {
-            double2 *ws = (double2 *)c0->d_ws;
-            switch (var) {
-                case V16x1:
-                    k_transmission_batch<16, 1, 2><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                    break;
-                case V16x2:
-                    k_transmission_batch<16, 2, 1><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                    break;
-                case V8x1:
-                    k_transmission_batch<8, 1, 2><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                    break;
-                default:
-                    k_transmission_batch<8, 4, 1><<<grid, NT, smem, st>>>(d_geo, d_jobs, njobs, d_E, ws, wstride, d_tj, d_info, d_counter);
-                    break;
-            }
-            if (cudaGetLastError() || cudaEventRecord(c0->ev1, st) ||
+            rc = launch_batch(k, grid, d_geo, d_jobs, njobs, d_E, (double2 *)c0->d_ws, k.ws, d_tj, d_info, d_counter, st);
+            if (rc || cudaEventRecord(c0->ev1, st) ||
                 cudaMemcpyAsync(tj.data(), d_tj, sizeof(double) * njobs, cudaMemcpyDeviceToHost, st) ||
                 cudaMemcpyAsync(info.data(), d_info, sizeof(int) * njobs, cudaMemcpyDeviceToHost, st) ||
                 cudaStreamSynchronize(st) || cudaEventElapsedTime(&ms, c0->ev0, c0->ev1))
@@ -1876,15 +1498,9 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
 
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const size_t smem = variant_smem(v, N);
+    const SweepKernel k = sweep_kernel(v, N);
     int occ = 1;
-    switch (v) {
-        case V16x1: rc = prep_kernel(k_transmission<16, 1, 2>, smem, &occ); break;
-        case V16x2: rc = prep_kernel(k_transmission<16, 2, 1>, smem, &occ); break;
-        case V8x1: rc = prep_kernel(k_transmission<8, 1, 2>, smem, &occ); break;
-        default: rc = prep_kernel(k_transmission<8, 4, 1>, smem, &occ); break;
-    }
-    if (rc) return rc;
+    if ((rc = prep_kernel(k.one, k.threads, k.smem, &occ))) return rc;
     const int grid = (int)std::min<size_t>(std::min<size_t>(njobs, (size_t)sms * occ), cap);
 
     const int nkv = std::max(N * nk, nk);
@@ -1900,21 +1516,7 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
     g.c2 = 2 * (g.delta * g.delta);
     g.V_L = V_L; g.V_R = V_R; g.eta = eta;
     g.lead_model = 0;
-    switch (v) {
-        case V16x1:
-            k_transmission<16, 1, 2><<<grid, NT, smem, st>>>(g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info);
-            break;
-        case V16x2:
-            k_transmission<16, 2, 1><<<grid, NT, smem, st>>>(g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info);
-            break;
-        case V8x1:
-            k_transmission<8, 1, 2><<<grid, NT, smem, st>>>(g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info);
-            break;
-        default:
-            k_transmission<8, 4, 1><<<grid, NT, smem, st>>>(g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info);
-            break;
-    }
-    CK(cudaGetLastError());
+    if ((rc = launch_one(k, grid, g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(tau_jobs, kw, nE, nk, d_tau);
     CK(cudaGetLastError());
     return NEGF_OK;

@@ -1,0 +1,54 @@
+// sweep_kernels.h -- the sweep kernels as the host code sees them: what each
+// launch needs, by kernel variant and basis size.  Private to the library.
+#pragma once
+#include "rgf_device.cuh"
+
+namespace negf {
+
+// One (problem, energy, k-point) job of a batch over several problems.
+struct BatchJob {
+    int prob, ie, ik, pad;
+};
+
+// A transmission kernel in its two forms, of one signature for every variant:
+//   one    (Geo, const double *energies, int nE, int njobs, double2 *ws, size_t wstride,
+//           double *tau_jobs, int *info_jobs): the nE * nk jobs of one problem, energy fastest
+//   batch  (const Geo *, const BatchJob *, int njobs, const double *energies, double2 *ws,
+//           size_t wstride, double *tau_jobs, int *info_jobs, int *counter): jobs of several
+//           problems, taken in order from a counter
+struct SweepKernel {
+    const void *one = nullptr, *batch = nullptr;
+    int threads = 0;
+    size_t smem = 0;  // dynamic shared memory for a basis of N
+    size_t ws = 0;    // workspace of one CTA in double2 for a basis of N
+};
+
+// The variants of negf_set_variant by basis size: (panel width NB, rows per
+// thread RPT, CTAs per SM).  Up to 256 plane waves two CTAs share an SM.
+enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, V8x1 = 3, VNONE = 4 };
+
+SweepKernel sweep_kernel(Variant v, int N);  // negf_transmission.cu
+
+struct RgfJob {
+    double e_re, e_im;  // complex energy of the solve, E + i*eta already added
+    double e_t;         // real energy of the transmission weights
+    int ik;             // k-point
+    int pad;
+    // WANT_A only: slice k of the output is cd * G_kk + ca * G_k,s Gamma_s G_k,s^H
+    // (s = the injecting lead's end slice, Gamma_s its open-channel widths)
+    double cd_re, cd_im, ca_re, ca_im;
+};
+
+enum { WANT_D = 1, WANT_F = 2, WANT_L = 4, WANT_A = 8, WANT_MIRROR = 16 };
+
+// k_rgf_slab's arguments: (Geo, const RgfJob *, int njobs, const double2 *Dexp, double2 *ws,
+// size_t wstride, double2 *slabs, size_t sstride, int want, double2 *out_first, double2 *out_last,
+// int *info_jobs); one CTA per job, six blocks of workspace.
+struct SlabKernel {
+    const void *fn = nullptr;
+    int threads = 0;
+    size_t smem = 0;
+};
+SlabKernel slab_kernel(Variant v, int N);     // negf_slab.cu
+
+}  // namespace negf
