@@ -303,9 +303,9 @@ bool variant_fits(int v, int N) {
     return (v == V16x1 && N <= NT) || (v == V16x2 && N <= 2 * NT) || (v == V8x4 && N <= 4 * NT) ||
            (v == V8x1 && N <= NT);
 }
-// Default variant of the transmission kernels: up to 256 plane waves the
-// 8-column panels in fours (8 x 1 x 2; at N = 69 7100 vs 5784 solves/s for
-// 16 x 1 x 2, at N = 221 194 vs 184).  The slab kernels keep pick_variant:
+// Default variant of the transmission kernels: up to 256 plane waves variant
+// 3, which is the register kernel up to RNMAX plane waves and the 8-column
+// panels in fours (8 x 1 x 2; at N = 221 194 vs 184 solves/s) above.  The slab kernels keep pick_variant:
 // their 8 x 1 x 2 build measured slower (N = 221: density 53.9 vs 55.2,
 // LDOS 47.3 vs 53.9 jobs/s; N = 69 LDOS 953 vs 1416).
 Variant transmission_variant(int N) { return N <= NT ? V8x1 : pick_variant(N); }
@@ -1052,11 +1052,14 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
     std::vector<int> info_all;
     double ms_all = 0;
     int rc = 0;
-    for (int v = V16x1; v <= V8x1 && !rc; ++v) {
+    // one launch per kernel, its problems in the order given
+    std::vector<const void *> kernels(nctx);
+    for (int p = 0; p < nctx; ++p) kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N).batch;
+    for (int first = 0; first < nctx && !rc; ++first) {
         std::vector<int> members;
         for (int p = 0; p < nctx; ++p)
-            if (ctx_variant(ctxs[p]) == v) members.push_back(p);
-        if (members.empty()) continue;
+            if (kernels[p] == kernels[first]) members.push_back(p);
+        if (members[0] != first) continue;  // launched already
         std::vector<Geo> geos;
         std::vector<BatchJob> jobs;
         std::vector<double> cost;
@@ -1078,7 +1081,7 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         std::vector<BatchJob> sorted(jobs.size());
         for (size_t q = 0; q < order.size(); ++q) sorted[q] = jobs[order[q]];
         const int njobs = (int)sorted.size();
-        const SweepKernel k = sweep_kernel((Variant)v, nmax);
+        const SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), nmax);
         int occ = 1;
         if ((rc = prep_kernel(k.batch, k.threads, k.smem, &occ))) break;
         const int grid = std::min(njobs, c0->num_sms * occ);

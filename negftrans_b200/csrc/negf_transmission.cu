@@ -124,7 +124,7 @@ SweepKernel sweep_kernel(Variant v, int N) {
         case V16x1: return make<16, 1, 2>(N);
         case V16x2: return make<16, 2, 1>(N);
         case V8x4: return make<8, 4, 1>(N);
-        case V8x1: return make<8, 1, 2>(N);
+        case V8x1: return N <= RNMAX ? register_kernel(N) : make<8, 1, 2>(N);
         default: return SweepKernel{};
     }
 }

@@ -212,7 +212,7 @@ __device__ inline Smem carve(unsigned char *base, int N) {
 // Self energies of the two leads for one job (grid.f90:284-289, 323-331) and
 // the transmission weights (grid.f90:354-360) at the real energy e_t.
 __device__ inline void job_vectors(const Geo &g, const Smem &s, double2 E, double e_t, int ik) {
-    for (int i = threadIdx.x; i < g.N; i += NT) {
+    for (int i = threadIdx.x; i < g.N; i += blockDim.x) {
         const double ax = g.ax[ik * g.N + i], ay = g.ay[ik * g.N + i];
         if (g.lead_model == 0) {
             double2 zl = make_double2(2.0 * (E.x - g.V_L) - ax * ax - ay * ay, 2.0 * E.y);

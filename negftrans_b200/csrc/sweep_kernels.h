@@ -28,6 +28,8 @@ struct SweepKernel {
 enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, V8x1 = 3, VNONE = 4 };
 
 SweepKernel sweep_kernel(Variant v, int N);  // negf_transmission.cu
+SweepKernel register_kernel(int N);          // negf_register.cu, up to RNMAX
+constexpr int RNMAX = 72;
 
 struct RgfJob {
     double e_re, e_im;  // complex energy of the solve, E + i*eta already added
