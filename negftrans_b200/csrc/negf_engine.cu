@@ -339,7 +339,7 @@ int launch_batch(const SweepKernel &k, int grid, const Geo *d_geo, const BatchJo
 
 // CTAs of the slab kernel resident per SM for this N.
 int resident_ctas(int N) {
-    const SlabKernel k = slab_kernel(pick_variant(N), N);
+    const SlabKernel k = slab_kernel(N);
     int occ = 1;
     if (k.fn) prep_kernel(k.fn, k.threads, k.smem, &occ);
     return occ;
@@ -365,9 +365,9 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
 int slab_launch(negf_ctx *c, const Geo &g, const RgfJob *d_jobs, int njobs, const double2 *d_D,
                 double2 *d_slabs, size_t sstride, int want, double2 *d_first, double2 *d_last,
                 int *d_info, cudaStream_t st) {
-    const SlabKernel k = slab_kernel(pick_variant(g.N), g.N);
+    const SlabKernel k = slab_kernel(g.N);
     if (!k.fn) return NEGF_ERR_UNSUPPORTED;
-    size_t wstride = 6 * (size_t)g.ld * g.N;
+    size_t wstride = k.blocks * (size_t)g.ld * g.N;
     int rc = ensure_ws(c, sizeof(double2) * wstride * njobs);
     if (rc) return rc;
     double2 *ws = (double2 *)c->d_ws;

@@ -190,13 +190,12 @@ SlabKernel make(int N) {
 
 }  // namespace
 
-SlabKernel slab_kernel(Variant v, int N) {
-    switch (v) {
-        case V16x1: return make<16, 1, 2>(N);
-        case V16x2: return make<16, 2, 1>(N);
-        case V8x4: return make<8, 4, 1>(N);
-        default: return SlabKernel{};
-    }
+SlabKernel slab_kernel(int N) {
+    if (N <= RNMAX) return register_slab_kernel(N);
+    if (N <= NT) return make<16, 1, 2>(N);
+    if (N <= 2 * NT) return make<16, 2, 1>(N);
+    if (N <= 4 * NT) return make<8, 4, 1>(N);
+    return SlabKernel{};
 }
 
 }  // namespace negf

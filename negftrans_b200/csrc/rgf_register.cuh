@@ -83,7 +83,7 @@ __device__ __forceinline__ void reg_pivot(double2 (&v)[NRL], unsigned free_rows,
 #pragma unroll
     for (int r = 0; r < PR; ++r) {
         int h = __double2hiint(cabs1(v[r]));
-        if (h >= 0x7ff80000) h = 0;  // a NaN ranks as a zero pivot
+        if ((unsigned)h >= 0x7ff80000u) h = 0;  // a NaN, of either sign, ranks as a zero pivot
         key = max(key, (free_rows >> r) & 1u ? (h & ~3) | r : -1);
     }
     // a lane without a candidate takes 1 / 1: no division by zero (slow path)
@@ -216,39 +216,58 @@ __device__ __forceinline__ void reg_eliminate(double2 (&a)[CPW][RPL], int N, con
 }
 
 // M = D_b - inv(previous block) in the registers, element on
-// element (grid.f90:236-333); the first block (b = Nz - 1) is D_b alone.
-// One column at a time: its PR gathers in flight, few registers beside a.
+// element (grid.f90:236-333); the first block of a sweep is D_b alone.  D_b is
+// generated, or read from the explicit blocks Dexp.  One column at a time: its
+// PR gathers in flight, few registers beside a.
 template <int PR, int CPW, int RPL, typename S>
 __device__ __forceinline__ void reg_form(double2 (&a)[CPW][RPL], const Geo &g, const S &s, const int *rho,
-                                         const int *kappa, const double2 *scale, int b, double2 E) {
+                                         const int *kappa, const double2 *scale, int b, double2 E, bool first,
+                                         const double2 *Dexp = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int N = g.N, Nz = g.Nz;
     const double2 *vs = g.vhat + (size_t)g.W * g.H * b + g.ngx + g.W * g.ngy;
+    const double2 *Dk = Dexp + (size_t)N * N * b;
 #pragma unroll
     for (int t = 0; t < CPW; ++t) {
         const int c = warp + RW * t;
         if (c < N) {
             const int kc = kappa[c];
-            const double2 *vc = vs - s.lin[kc];
             double2 d[PR];
 #pragma unroll
-            for (int r = 0; r < PR; ++r)
-                d[r] = (lane + 32 * r < N) ? __ldg(vc + s.lin[rho[lane + 32 * r]]) : make_double2(0.0, 0.0);
+            for (int r = 0; r < PR; ++r) {
+                const int m = lane + 32 * r < N ? rho[lane + 32 * r] : -1;
+                d[r] = m < 0 ? make_double2(0.0, 0.0) : Dexp ? Dk[m + (size_t)N * kc] : __ldg(vs + (s.lin[m] - s.lin[kc]));
+            }
 #pragma unroll
             for (int r = 0; r < PR; ++r)
                 if (lane + 32 * r < N) {
                     const int m = rho[lane + 32 * r];
-                    double2 x;
-                    if (m != kc) x = make_double2(-d[r].x * g.c2, -d[r].y * g.c2);
-                    else {  // the diagonal and the lead terms of the end blocks
-                        x = make_double2((-(d[r].x + s.kin[m]) + E.x) * g.c2 - 2.0, (-d[r].y + E.y) * g.c2);
-                        if (b == 0) x = zadd(x, s.sigL[m]);
-                        if (b == Nz - 1) x = zadd(x, s.sigR[m]);
+                    double2 x = d[r];
+                    if (!Dexp) {
+                        if (m != kc) x = make_double2(-d[r].x * g.c2, -d[r].y * g.c2);
+                        else {  // the diagonal and the lead terms of the end blocks
+                            x = make_double2((-(d[r].x + s.kin[m]) + E.x) * g.c2 - 2.0, (-d[r].y + E.y) * g.c2);
+                            if (b == 0) x = zadd(x, s.sigL[m]);
+                            if (b == Nz - 1) x = zadd(x, s.sigR[m]);
+                        }
                     }
-                    a[t][r] = b == Nz - 1 ? x : zfms(scale[lane + 32 * r], a[t][r], x);
+                    a[t][r] = first ? x : zfms(scale[lane + 32 * r], a[t][r], x);
                 }
         }
     }
+}
+
+// The maps of the inverse, from those of the block (parity sp): the CTA's
+// threads together, before the next block is formed.
+template <typename S>
+__device__ __forceinline__ void reg_remap(S &s, int N, int sp) {
+    if (threadIdx.x < N) {
+        const int j = threadIdx.x, p = s.prow[j], c = s.cst[sp][j], m = s.rho[sp][p];
+        s.rho[sp ^ 1][p] = j;
+        s.kappa[sp ^ 1][(c >> 8) * RW + (c & 255)] = m;
+        s.cst[sp ^ 1][m] = c;
+    }
+    __syncthreads();
 }
 
 // One F-mode sweep and its transmission trace (math_kernel.f90:81-128,
@@ -284,7 +303,7 @@ __device__ double reg_transmission_job(const Geo &g, S &s, double e, int ik, int
         }
     int sp = 0;
     for (int b = Nz - 1; b >= 0; --b) {
-        reg_form<PR>(a, g, s, s.rho[sp], s.kappa[sp], s.scale[sp ^ 1], b, E);
+        reg_form<PR>(a, g, s, s.rho[sp], s.kappa[sp], s.scale[sp ^ 1], b, E, b == Nz - 1);
         // the code of this job's row count: no tests of slots inside the steps
         each_slot<RPL - PR + 1>([&](auto x) {
             if (nrl == PR + x.v || (x.v == 0 && nrl < PR)) {
@@ -292,13 +311,7 @@ __device__ double reg_transmission_job(const Geo &g, S &s, double e, int ik, int
                 reg_keep<x.v>();
             }
         });
-        if (tid < N) {
-            const int p = s.prow[tid], c = s.cst[sp][tid], m = s.rho[sp][p];
-            s.rho[sp ^ 1][p] = tid;
-            s.kappa[sp ^ 1][(c >> 8) * RW + (c & 255)] = m;
-            s.cst[sp ^ 1][m] = c;
-        }
-        __syncthreads();
+        reg_remap(s, N, sp);
         sp ^= 1;
     }
     // tau = sum_ij gamma_L,i gamma_R,j |2 dz^2 G_{Nz,1}(i,j)|^2   grid.f90:362-383

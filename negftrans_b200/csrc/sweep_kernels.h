@@ -45,12 +45,14 @@ enum { WANT_D = 1, WANT_F = 2, WANT_L = 4, WANT_A = 8, WANT_MIRROR = 16 };
 
 // k_rgf_slab's arguments: (Geo, const RgfJob *, int njobs, const double2 *Dexp, double2 *ws,
 // size_t wstride, double2 *slabs, size_t sstride, int want, double2 *out_first, double2 *out_last,
-// int *info_jobs); one CTA per job, six blocks of workspace.
+// int *info_jobs); one CTA per job.
 struct SlabKernel {
     const void *fn = nullptr;
     int threads = 0;
     size_t smem = 0;
+    int blocks = 6;  // workspace of a job in blocks of round_up(N, 8) x N
 };
-SlabKernel slab_kernel(Variant v, int N);     // negf_slab.cu
+SlabKernel slab_kernel(int N);                // negf_slab.cu
+SlabKernel register_slab_kernel(int N);       // negf_register_slab.cu, up to RNMAX
 
 }  // namespace negf

@@ -8,7 +8,7 @@ import pytest
 
 from negftrans_b200 import workloads as W
 from negftrans_b200 import prepare as P
-from negftrans_b200.negf import Engine, transmission_batch
+from negftrans_b200.negf import Engine, GreensFunction_tri_solver, transmission_batch
 
 pytestmark = pytest.mark.gpu
 RTOL, ATOL = 1e-9, 1e-12
@@ -54,3 +54,57 @@ def test_batch_over_every_small_kernel(oracle):
     for p, t in zip(probs, tau):
         ref, _ = oracle.transmission_jobs(p[1], E, nthreads=4)
         np.testing.assert_allclose(t, ref, rtol=RTOL, atol=ATOL)
+
+
+# the register slab kernels: tiles of 8, warps' columns of 12, rows of 32
+@pytest.mark.parametrize("N,Nz", [(1, 3), (2, 2), (8, 4), (23, 2), (24, 5), (25, 3), (47, 2), (48, 4), (49, 3), (65, 3),
+                                  (71, 2), (72, 5), (73, 3)])
+def test_small_tri_solves(oracle, N, Nz):
+    rng = np.random.default_rng(100 * N + Nz)
+    D = rng.standard_normal((N, N, Nz)) + 1j * rng.standard_normal((N, N, Nz))
+    D[np.arange(N), np.arange(N)] += 4.0 * np.sqrt(N)
+    D[0, 0, 0] = 0.0  # the first column's natural pivot is no pivot
+    D = np.asfortranarray(D)
+    ref, rinfo = oracle.tri_solver(D, "DFL")
+    got, info = GreensFunction_tri_solver(D, "DFL")
+    assert info == rinfo
+    if N == 1:  # the left sweep's first block is singular: reported, not trusted
+        assert info == 1
+        return
+    assert info == 0
+    for key in "DFL":
+        scale = np.max(np.abs(ref[key]))
+        assert np.max(np.abs(got[key] - ref[key])) <= RTOL * scale
+        only, _ = GreensFunction_tri_solver(D, key)  # alone, the other planes' passes left out
+        assert np.max(np.abs(only[key] - ref[key])) <= RTOL * scale
+
+
+@pytest.mark.parametrize("N,nk", [(20, 2), (48, 1), (69, 1), (72, 1)])
+@pytest.mark.parametrize("bias", [1e-5, -1e-5])
+def test_small_biased_density(oracle, N, nk, bias):
+    args, op, pr = cut_problem(oracle, N, nz=4, nk=nk)
+    a = pr.atomic
+    ref, _ = oracle.density_neq(op, 3, 4, pr.min_V, a.MU + bias, a.MU, a.GAP, a.TEMPERATURE)
+    with Engine(*args) as eng:
+        dm, info = eng.density_neq(3, 4, pr.min_V, a.MU + bias, a.MU, a.GAP, a.TEMPERATURE)
+    assert info == 0
+    assert np.max(np.abs(dm - ref)) <= RTOL * np.max(np.abs(ref))
+
+
+def test_nan_and_singular_blocks_are_reported(oracle):
+    """A NaN energy and a singular block end as an info, with the other jobs intact."""
+    args, op, pr = cut_problem(oracle, 45, nz=3)
+    E = P.transmission_energies(pr.atomic, 16)[2:5].copy()
+    ref, _ = oracle.transmission_jobs(op, E, nthreads=4)
+    bad = E.copy()
+    bad[1] = np.nan
+    with Engine(*args) as eng:
+        tau, info = eng.transmission(bad)
+        assert info > 0 and eng.last_stats.n_singular == 1 and eng.last_stats.first_bad_job == 1
+    np.testing.assert_allclose(tau[[0, 2]], ref[[0, 2]], rtol=RTOL, atol=ATOL)
+    for N in (5, 30, 60):
+        D = np.asfortranarray(np.zeros((N, N, 3), np.complex128))
+        D[np.arange(N), np.arange(N)] = 3.0
+        D[:, N // 2, 2] = 0.0  # a zero column in the block the right sweep starts from
+        _, info = GreensFunction_tri_solver(D, "DF")
+        assert info == N // 2 + 1
