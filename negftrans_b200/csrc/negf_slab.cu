@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(NT, MINB)
 
 template <int NB, int RPT, int MINB>
 SlabKernel make(int N) {
-    return SlabKernel{(const void *)k_rgf_slab<NB, RPT, MINB>, NT, smem_bytes<NB>(N)};
+    return SlabKernel{(const void *)k_rgf_slab<NB, RPT, MINB>, NT, smem_bytes<NB, RPT>(N)};
 }
 
 }  // namespace

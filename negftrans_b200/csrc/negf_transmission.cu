@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(NT, MINB)
 template <int NB, int RPT, int MINB>
 SweepKernel make(int N) {
     return SweepKernel{(const void *)k_transmission<NB, RPT, MINB>, (const void *)k_transmission_batch<NB, RPT, MINB>,
-                       NT, smem_bytes<NB>(N), 4 * (size_t)round_up(N, 8) * N};
+                       NT, smem_bytes<NB, RPT>(N), 4 * (size_t)round_up(N, 8) * N};
 }
 
 }  // namespace

@@ -165,11 +165,12 @@ struct Smem {
 
 __host__ __device__ inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-template <int NB>
+template <int NB, int RPT>
 __host__ __device__ inline size_t smem_bytes(int N) {
     int ldw = round_up(N, CM);
     size_t big = (size_t)NB * ldw + (size_t)NB * NB;         // sub-panel a + 16x16 block
     size_t trail = 32 * (size_t)(BP + AP);                    // rank-32 update: gathered rows + W tile
+    if (RPT > 1) trail *= 2;                                  // trailing_update_wide keeps two of each
     size_t gemm = 2 * (size_t)KC * (AP + BP);
     if (trail > big) big = trail;
     if (gemm > big) big = gemm;
@@ -502,7 +503,7 @@ __device__ inline double block_sum(double v, const Smem &s) {
 // steps on the other columns, so one pass over the matrix applies KMAX
 // elimination steps.  W tiles are staged from global memory with cp.async;
 // W and the gathered pivot rows feed DMMA warp tiles.
-template <int KMAX, bool PREFETCH = false>
+template <int KMAX>
 __device__ inline void trailing_update(double2 *__restrict__ A, int N, int ld, int k0, int nbt,
                                        const Smem &s) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -550,20 +551,6 @@ __device__ inline void trailing_update(double2 *__restrict__ A, int N, int ld, i
                 cp_async16(sW + kk * AP + r, A + (v ? (i + (size_t)ld * (k0 + kk)) : 0), v);
             }
             cp_async_commit();
-            // large blocks (one CTA per SM): start the warp's C tile on its way
-            // from DRAM into L2 while W arrives (slower for the 2-CTA variants)
-            if (PREFETCH && (I0 + wm0 < N) && (J0 + wn0 < nrest)) {
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int i = I0 + wm0 + 8 * m + (lane >> 2);
-#pragma unroll
-                    for (int n = 0; n < 2; ++n)
-#pragma unroll
-                        for (int e = 0; e < 2; ++e)
-                            if (i < N && cv[n][e])
-                                asm volatile("prefetch.global.L2 [%0];" ::"l"(A + i + (size_t)ld * col[n][e]));
-                }
-            }
             cp_async_wait<0>();
             __syncthreads();
             if ((I0 + wm0 < N) && (J0 + wn0 < nrest)) {
@@ -599,6 +586,104 @@ __device__ inline void trailing_update(double2 *__restrict__ A, int N, int ld, i
             __syncthreads();
         }
     }
+}
+
+// The same update for the variants of one CTA per SM (RPT > 1), where nothing
+// else covers a tile's loads: the 64 x 64 tiles run as one pipeline, rows
+// fastest.  While a tile multiplies, the next one's W tile (and, at a new
+// column tile, its pivot rows) arrive by cp.async in the other buffer and its
+// old values in registers, so a tile costs its DMMAs and one barrier.  The
+// loads are dealt over the first half of the k steps: issued together they
+// hold the warps' DMMAs back while they pass the load unit, issued later they
+// are not back in time.  Bound by the DMMA rate, then by the block's own
+// traffic (it exceeds L2).
+template <int KMAX>
+__device__ inline void trailing_update_wide(double2 *__restrict__ A, int N, int ld, int k0, int nbt, const Smem &s) {
+    static_assert(KMAX == 32 && CM == 64 && CN == 64 && NT == 256, "8 k steps, 8 copies of each kind per thread and tile");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm0 = (warp >> 2) * WM, wn0 = (warp & 3) * WN;
+    const int nrest = N - nbt;
+    double2 *sB = s.big;                    // [2][KMAX][BP] pivot rows of a column tile
+    double2 *sW = s.big + 2 * KMAX * BP;    // [2][KMAX][AP] rows of the panel
+    const int nti = (N + CM - 1) / CM, ntj = (nrest + CN - 1) / CN;
+    auto column = [&](int jr) { return A + (size_t)ld * (jr < k0 ? jr : jr + nbt); };
+    // part u of the copies of tile (ti, tj): W into buffer bw, the pivot rows
+    auto stage = [&](int u, int ti, int tj, int bw) {
+        const int kk = (tid + NT * u) / CM, r = tid % CM, i = ti * CM + r;
+        const bool v = (kk < nbt) && (i < N);
+        cp_async16(sW + (bw * KMAX + kk) * AP + r, A + (v ? (i + (size_t)ld * (k0 + kk)) : 0), v);
+        if (ti == 0) {
+            const int kb = tid % KMAX, jt = (tid + NT * u) / KMAX, jr = tj * CN + jt;
+            const bool vb = (kb < nbt) && (jr < nrest);
+            cp_async16(sB + ((tj & 1) * KMAX + kb) * BP + jt, vb ? column(jr) + s.prow[k0 + kb] : A, vb);
+        }
+    };
+    double2 c[4][2][2];
+    auto load = [&](int m, int n, int ti, int tj) {
+        const int i = ti * CM + wm0 + 8 * m + (lane >> 2);
+        const bool rv = (i < N) && !s.inP[i];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int jr = tj * CN + wn0 + 8 * n + 2 * (lane & 3) + e;
+            c[m][n][e] = make_double2(0.0, 0.0);
+            if (rv && jr < nrest) c[m][n][e] = column(jr)[i];
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        stage(u, 0, 0, 0);
+        load(u / 2, u % 2, 0, 0);
+    }
+    cp_async_commit();
+    for (int t = 0, ti = 0, tj = 0; t < nti * ntj; ++t) {
+        const int bw = t & 1;
+        int ni = ti + 1, nj = tj;
+        if (ni == nti) { ni = 0; ++nj; }
+        const bool more = nj < ntj, active = (ti * CM + wm0 < N) && (tj * CN + wn0 < nrest);
+        cp_async_wait<0>();
+        __syncthreads();  // this tile's operands are here; the tile before is done with the other buffers
+        WarpAcc acc;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    acc.re[m][n][e] = c[m][n][e].x;
+                    acc.im[m][n][e] = c[m][n][e].y;
+                }
+        const double2 *w = sW + bw * KMAX * AP, *b = sB + (tj & 1) * KMAX * BP;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (more && u < 4) {
+                load(u, 0, ni, nj);
+                load(u, 1, ni, nj);
+                stage(2 * u, ni, nj, bw ^ 1);
+                stage(2 * u + 1, ni, nj, bw ^ 1);
+            }
+            if (active && 4 * u < nbt) acc.step(w, AP, wm0, b, BP, wn0, 4 * u, lane);
+        }
+        cp_async_commit();
+        if (active) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int jr = tj * CN + wn0 + 8 * n + 2 * (lane & 3) + e;
+                    if (jr < nrest) {
+                        double2 *col = column(jr);
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {
+                            const int i = ti * CM + wm0 + 8 * m + (lane >> 2);
+                            if (i < N) col[i] = make_double2(acc.re[m][n][e], acc.im[m][n][e]);
+                        }
+                    }
+                }
+        }
+        ti = ni;
+        tj = nj;
+    }
+    __syncthreads();
 }
 
 // Gauss-Jordan elimination of the columns [kb, kb+nbe) of a register panel
@@ -840,7 +925,10 @@ __device__ int gj_invert_pair(double2 *__restrict__ A, int N, int ld, const Smem
             }
         }
         __syncthreads();
-        if (nbt < N) trailing_update<2 * NB>(A, N, ld, k0, nbt, s);
+        if (nbt < N) {
+            if constexpr (RPT > 1) trailing_update_wide<2 * NB>(A, N, ld, k0, nbt, s);
+            else trailing_update<2 * NB>(A, N, ld, k0, nbt, s);
+        }
         __syncthreads();
         if (tid < nbt) s.inP[s.prow[k0 + tid]] = 0;
         __syncthreads();
@@ -942,7 +1030,10 @@ __device__ int gj_invert_multi(double2 *__restrict__ A, int N, int ld, const Sme
             }
             __syncthreads();
         }
-        if (nbt < N) trailing_update<P * NB, (RPT >= 4)>(A, N, ld, k0, nbt, s);
+        if (nbt < N) {
+            if constexpr (RPT > 1) trailing_update_wide<P * NB>(A, N, ld, k0, nbt, s);
+            else trailing_update<P * NB>(A, N, ld, k0, nbt, s);
+        }
         __syncthreads();
         if (tid < nbt) s.inP[s.prow[k0 + tid]] = 0;
         __syncthreads();
