@@ -13,13 +13,14 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libnegfgpu.so")
 DRIVER = os.path.join(PKG, "negftrans")   # the main.f90-style executable
-SOURCES = ["negf_engine.cu", "negf_transmission.cu", "negf_slab.cu", "negf_register.cu", "negf_register_slab.cu", "negf_host.cpp", "mlp.cu", "negf_mixed.cu"]
-HEADERS = ["rgf_device.cuh", "rgf_register.cuh", "sweep_kernels.h", "engine_internal.h", "tc_umma.cuh", "mixed_device.cuh"]
+SOURCES = ["negf_engine.cu", "negf_transmission.cu", "negf_slab.cu", "negf_register.cu", "negf_register_slab.cu", "negf_panel.cu", "negf_host.cpp", "mlp.cu", "negf_mixed.cu"]
+HEADERS = ["rgf_device.cuh", "rgf_register.cuh", "rgf_panel.cuh", "sweep_kernels.h", "engine_internal.h", "tc_umma.cuh", "mixed_device.cuh"]
 # private headers each source includes
 DEPS = {"negf_engine.cu": ("rgf_device.cuh", "sweep_kernels.h", "engine_internal.h"),
         "negf_transmission.cu": ("rgf_device.cuh", "sweep_kernels.h"),
         "negf_register.cu": ("rgf_device.cuh", "rgf_register.cuh", "sweep_kernels.h"),
         "negf_register_slab.cu": ("rgf_device.cuh", "rgf_register.cuh", "sweep_kernels.h"),
+        "negf_panel.cu": ("rgf_device.cuh", "rgf_register.cuh", "rgf_panel.cuh", "sweep_kernels.h"),
         "negf_slab.cu": ("rgf_device.cuh", "sweep_kernels.h"),
         "negf_mixed.cu": ("rgf_device.cuh", "engine_internal.h", "tc_umma.cuh", "mixed_device.cuh")}
 PUBLIC_HEADERS = ["negf_gpu.h", "negf_mlp.h"]

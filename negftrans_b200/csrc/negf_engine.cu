@@ -301,14 +301,13 @@ Variant pick_variant(int N) {
 }
 bool variant_fits(int v, int N) {
     return (v == V16x1 && N <= NT) || (v == V16x2 && N <= 2 * NT) || (v == V8x4 && N <= 4 * NT) ||
-           (v == V8x1 && N <= NT);
+           (v == VCHIP && N <= NT);
 }
-// Default variant of the transmission kernels: up to 256 plane waves variant
-// 3, which is the register kernel up to RNMAX plane waves and the 8-column
-// panels in fours (8 x 1 x 2; at N = 221 194 vs 184 solves/s) above.  The slab kernels keep pick_variant:
+// Default variant of the transmission kernels: variant 3 up to PNMAX plane waves
+// (sweep_kernel says which kernel that is), then the narrowest that holds N.  The slab kernels keep pick_variant:
 // their 8 x 1 x 2 build measured slower (N = 221: density 53.9 vs 55.2,
 // LDOS 47.3 vs 53.9 jobs/s; N = 69 LDOS 953 vs 1416).
-Variant transmission_variant(int N) { return N <= NT ? V8x1 : pick_variant(N); }
+Variant transmission_variant(int N) { return N <= PNMAX ? VCHIP : pick_variant(N); }
 Variant ctx_variant(const negf_ctx *c) {
     return (c->variant >= 0 && variant_fits(c->variant, c->N)) ? (Variant)c->variant : transmission_variant(c->N);
 }
@@ -321,19 +320,67 @@ int prep_kernel(const void *fn, int threads, size_t smem, int *occ) {
     return 0;
 }
 
+// How a sweep kernel runs njobs jobs: CTAs per job (a thread-block cluster) and
+// CTAs in all.
+struct Shape {
+    int team = 1, grid = 0;
+};
+
+cudaLaunchConfig_t sweep_config(const SweepKernel &k, Shape sh, cudaLaunchAttribute *at, cudaStream_t st) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(sh.grid);
+    lc.blockDim = dim3(k.threads);
+    lc.dynamicSmemBytes = k.smem;
+    lc.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = sh.team;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = sh.team > 1 ? 1 : 0;
+    return lc;
+}
+
+// Readies fn (one of k's two forms) and shapes its launch for njobs jobs, at
+// most max_teams of them at once.  The team is the largest that still runs
+// every job at once: a smaller one would leave SMs idle, a larger one would
+// make jobs wait, and a team's time falls by less than its size.
+int shape_sweep(const void *fn, const SweepKernel &k, int sms, int njobs, size_t max_teams, Shape *sh) {
+    int occ = 1;
+    int rc = prep_kernel(fn, k.threads, k.smem, &occ);
+    if (rc) return rc;
+    size_t teams = (size_t)sms * occ;
+    for (sh->team = k.team; sh->team > 1; sh->team /= 2) {
+        cudaLaunchAttribute at{};
+        sh->grid = sh->team;
+        const cudaLaunchConfig_t lc = sweep_config(k, *sh, &at, nullptr);
+        int most = 0;
+        CK(cudaOccupancyMaxActiveClusters(&most, fn, &lc));
+        if (njobs <= most) {
+            teams = (size_t)most;
+            break;
+        }
+    }
+    sh->grid = (int)std::min({(size_t)njobs, teams, max_teams}) * sh->team;
+    return 0;
+}
+
 // The one-problem form of k on njobs jobs.
-int launch_one(const SweepKernel &k, int grid, Geo g, const double *d_E, int nE, int njobs, double2 *ws, size_t wstride,
+int launch_one(const SweepKernel &k, Shape sh, Geo g, const double *d_E, int nE, int njobs, double2 *ws, size_t wstride,
                double *d_tau_jobs, int *d_info, cudaStream_t st) {
     void *args[] = {&g, &d_E, &nE, &njobs, &ws, &wstride, &d_tau_jobs, &d_info};
-    CK(cudaLaunchKernel(k.one, dim3(grid), dim3(k.threads), args, k.smem, st));
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t lc = sweep_config(k, sh, &at, st);
+    CK(cudaLaunchKernelExC(&lc, k.one, args));
     return 0;
 }
 
 // The batch form of k.
-int launch_batch(const SweepKernel &k, int grid, const Geo *d_geo, const BatchJob *d_jobs, int njobs, const double *d_E,
+int launch_batch(const SweepKernel &k, Shape sh, const Geo *d_geo, const BatchJob *d_jobs, int njobs, const double *d_E,
                  double2 *ws, size_t wstride, double *d_tj, int *d_info, int *d_counter, cudaStream_t st) {
     void *args[] = {&d_geo, &d_jobs, &njobs, &d_E, &ws, &wstride, &d_tj, &d_info, &d_counter};
-    CK(cudaLaunchKernel(k.batch, dim3(grid), dim3(k.threads), args, k.smem, st));
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t lc = sweep_config(k, sh, &at, st);
+    CK(cudaLaunchKernelExC(&lc, k.batch, args));
     return 0;
 }
 
@@ -350,13 +397,12 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
     const int njobs = nE * c->nk;
     const Variant v = ctx_variant(c);
     if (v == VNONE) return NEGF_ERR_UNSUPPORTED;
-    const SweepKernel k = sweep_kernel(v, c->N);
-    int occ = 1;
-    int rc = prep_kernel(k.one, k.threads, k.smem, &occ);
+    const SweepKernel k = sweep_kernel(v, c->N, 2 * (int64_t)njobs <= c->num_sms);
+    Shape sh;
+    int rc = shape_sweep(k.one, k, c->num_sms, njobs, SIZE_MAX, &sh);
     if (rc) return rc;
-    const int grid = std::min(njobs, c->num_sms * occ);
-    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * grid))) return rc;
-    if ((rc = launch_one(k, grid, make_geo(c), d_E, nE, njobs, (double2 *)c->d_ws, k.ws, d_tau_jobs, d_info, st))) return rc;
+    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * (sh.grid / sh.team)))) return rc;
+    if ((rc = launch_one(k, sh, make_geo(c), d_E, nE, njobs, (double2 *)c->d_ws, k.ws, d_tau_jobs, d_info, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(d_tau_jobs, c->d_kw, nE, c->nk, d_tau);
     CK(cudaGetLastError());
     return 0;
@@ -658,7 +704,7 @@ int negf_transmission(negf_ctx *c, const double *energies, int32_t nE, int32_t p
 }
 
 int negf_set_variant(negf_ctx *c, int32_t variant) {
-    if (!c || variant < -1 || variant > V8x1) return NEGF_ERR_ARG;
+    if (!c || variant < -1 || variant > VCHIP) return NEGF_ERR_ARG;
     if (variant >= 0 && !variant_fits(variant, c->N)) return NEGF_ERR_UNSUPPORTED;
     c->variant = variant;
     return NEGF_OK;
@@ -670,7 +716,7 @@ int negf_autotune(negf_ctx *c, const double *energies, int32_t nE, int32_t *chos
     double best = -1.0;
     int bv = -1;
     const int keep = c->variant;
-    for (int v = V16x1; v <= V8x1; ++v) {
+    for (int v = V16x1; v <= VCHIP; ++v) {
         if (rates) rates[v] = 0.0;
         if (!variant_fits(v, c->N)) continue;
         c->variant = v;
@@ -982,12 +1028,11 @@ int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const
     if (var == VNONE) return NEGF_ERR_UNSUPPORTED;
     std::vector<BatchJob> jobs(njobs);
     for (int q = 0; q < njobs; ++q) jobs[q] = BatchJob{0, ie[q], ik[q], 0};
-    const SweepKernel k = sweep_kernel(var, c->N);
-    int occ = 1;
-    int rc = prep_kernel(k.batch, k.threads, k.smem, &occ);
+    const SweepKernel k = sweep_kernel(var, c->N, 2 * (int64_t)njobs <= c->num_sms);
+    Shape sh;
+    int rc = shape_sweep(k.batch, k, c->num_sms, njobs, SIZE_MAX, &sh);
     if (rc) return rc;
-    const int grid = std::min(njobs, c->num_sms * occ);
-    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * grid))) return rc;
+    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * (sh.grid / sh.team)))) return rc;
     Geo g = make_geo(c);
     Geo *d_geo = nullptr;
     BatchJob *d_jobs = nullptr;
@@ -1004,7 +1049,7 @@ int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const
                 cudaMemsetAsync(d_counter, 0, sizeof(int), st) || cudaEventRecord(c->ev0, st)))
         rc = NEGF_ERR_CUDA;
     if (!rc) {
-        rc = launch_batch(k, grid, d_geo, d_jobs, njobs, d_E, (double2 *)c->d_ws, k.ws, d_tj, d_info, d_counter, st);
+        rc = launch_batch(k, sh, d_geo, d_jobs, njobs, d_E, (double2 *)c->d_ws, k.ws, d_tj, d_info, d_counter, st);
         if (rc || cudaEventRecord(c->ev1, st) ||
             cudaMemcpyAsync(h_tau, d_tj, sizeof(double) * njobs, cudaMemcpyDeviceToHost, st) ||
             cudaMemcpyAsync(h_info, d_info, sizeof(int) * njobs, cudaMemcpyDeviceToHost, st) ||
@@ -1052,9 +1097,22 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
     std::vector<int> info_all;
     double ms_all = 0;
     int rc = 0;
-    // one launch per kernel, its problems in the order given
+    // One launch per kernel, its problems in the order given.  The middle sizes
+    // (RNMAX < N <= PNMAX, chosen by N) stay together: with bases on both sides
+    // of NT, or few jobs, all of them run in the panel kernel, since a second
+    // launch would wait for the first one's last sweep (48 problems of 180-263
+    // plane waves, 576 sweeps: 272 ms in two launches, 143 in one).
+    bool wide = false;
+    int64_t middle = 0;
+    for (int p = 0; p < nctx; ++p) {
+        const negf_ctx *c = ctxs[p];
+        if (ctx_variant(c) != VCHIP || c->N <= RNMAX) continue;
+        wide = wide || c->N > NT;
+        middle += (int64_t)nE * c->nk;
+    }
+    const bool few = wide || 2 * middle <= c0->num_sms;
     std::vector<const void *> kernels(nctx);
-    for (int p = 0; p < nctx; ++p) kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N).batch;
+    for (int p = 0; p < nctx; ++p) kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, few).batch;
     for (int first = 0; first < nctx && !rc; ++first) {
         std::vector<int> members;
         for (int p = 0; p < nctx; ++p)
@@ -1081,11 +1139,10 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         std::vector<BatchJob> sorted(jobs.size());
         for (size_t q = 0; q < order.size(); ++q) sorted[q] = jobs[order[q]];
         const int njobs = (int)sorted.size();
-        const SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), nmax);
-        int occ = 1;
-        if ((rc = prep_kernel(k.batch, k.threads, k.smem, &occ))) break;
-        const int grid = std::min(njobs, c0->num_sms * occ);
-        if ((rc = ensure_ws(c0, sizeof(double2) * k.ws * grid))) break;
+        const SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), nmax, few);
+        Shape sh;
+        if ((rc = shape_sweep(k.batch, k, c0->num_sms, njobs, SIZE_MAX, &sh))) break;
+        if ((rc = ensure_ws(c0, sizeof(double2) * k.ws * (sh.grid / sh.team)))) break;
         Geo *d_geo = nullptr;
         BatchJob *d_jobs = nullptr;
         double *d_tj = nullptr;
@@ -1108,7 +1165,7 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
                 rc = NEGF_ERR_CUDA;
         }
         if (!rc) {
-            rc = launch_batch(k, grid, d_geo, d_jobs, njobs, d_E, (double2 *)c0->d_ws, k.ws, d_tj, d_info, d_counter, st);
+            rc = launch_batch(k, sh, d_geo, d_jobs, njobs, d_E, (double2 *)c0->d_ws, k.ws, d_tj, d_info, d_counter, st);
             if (rc || cudaEventRecord(c0->ev1, st) ||
                 cudaMemcpyAsync(tj.data(), d_tj, sizeof(double) * njobs, cudaMemcpyDeviceToHost, st) ||
                 cudaMemcpyAsync(info.data(), d_info, sizeof(int) * njobs, cudaMemcpyDeviceToHost, st) ||
@@ -1501,10 +1558,9 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
 
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const SweepKernel k = sweep_kernel(v, N);
-    int occ = 1;
-    if ((rc = prep_kernel(k.one, k.threads, k.smem, &occ))) return rc;
-    const int grid = (int)std::min<size_t>(std::min<size_t>(njobs, (size_t)sms * occ), cap);
+    const SweepKernel k = sweep_kernel(v, N, 2 * njobs <= (size_t)sms);
+    Shape sh;
+    if ((rc = shape_sweep(k.one, k, sms, (int)njobs, cap, &sh))) return rc;
 
     const int nkv = std::max(N * nk, nk);
     k_noalloc_kvectors<<<(nkv + 255) / 256, 256, 0, st>>>(d_nx, d_ny, d_kpt, N, nk, Lx, Ly, ax, ay, kw);
@@ -1519,7 +1575,7 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
     g.c2 = 2 * (g.delta * g.delta);
     g.V_L = V_L; g.V_R = V_R; g.eta = eta;
     g.lead_model = 0;
-    if ((rc = launch_one(k, grid, g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info, st))) return rc;
+    if ((rc = launch_one(k, sh, g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(tau_jobs, kw, nE, nk, d_tau);
     CK(cudaGetLastError());
     return NEGF_OK;

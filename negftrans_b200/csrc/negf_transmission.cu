@@ -119,12 +119,14 @@ SweepKernel make(int N) {
 
 }  // namespace
 
-SweepKernel sweep_kernel(Variant v, int N) {
+SweepKernel sweep_kernel(Variant v, int N, bool few) {
     switch (v) {
         case V16x1: return make<16, 1, 2>(N);
         case V16x2: return make<16, 2, 1>(N);
         case V8x4: return make<8, 4, 1>(N);
-        case V8x1: return N <= RNMAX ? register_kernel(N) : make<8, 1, 2>(N);
+        case VCHIP:
+            if (N <= RNMAX) return register_kernel(N);
+            return few || N > NT ? panel_kernel(N) : make<8, 1, 2>(N);
         default: return SweepKernel{};
     }
 }

@@ -20,16 +20,26 @@ struct SweepKernel {
     const void *one = nullptr, *batch = nullptr;
     int threads = 0;
     size_t smem = 0;  // dynamic shared memory for a basis of N
-    size_t ws = 0;    // workspace of one CTA in double2 for a basis of N
+    size_t ws = 0;    // workspace of one CTA (team) in double2 for a basis of N
+    int team = 1;     // most CTAs (a thread-block cluster) that can share a job
 };
 
-// The variants of negf_set_variant by basis size: (panel width NB, rows per
-// thread RPT, CTAs per SM).  Up to 256 plane waves two CTAs share an SM.
-enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, V8x1 = 3, VNONE = 4 };
+// The variants of negf_set_variant.  0 .. 2 keep the block in global memory:
+// (panel width NB, rows per thread RPT, CTAs per SM), two CTAs per SM up to 256
+// plane waves.  3 is the family below, by basis size and number of jobs.
+enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, VCHIP = 3, VNONE = 4 };
 
-SweepKernel sweep_kernel(Variant v, int N);  // negf_transmission.cu
+// The kernel of a variant for a basis of N.  Variant 3: the block in registers
+// up to RNMAX; above, panels in registers and teams of CTAs if the jobs are
+// few (at most one per two SMs: nine jobs of N = 221, N_z = 160, 175 -> 86 ms in
+// teams of eight) or N > 256 (the next variant takes a whole SM as
+// well, at two rows per thread); otherwise 8 x 1 x 2, whose two jobs per SM
+// cover each other's pivots (N = 221: 920 us of an SM per slice and job, the
+// panel kernel 1240).
+SweepKernel sweep_kernel(Variant v, int N, bool few);  // negf_transmission.cu
 SweepKernel register_kernel(int N);          // negf_register.cu, up to RNMAX
-constexpr int RNMAX = 72;
+SweepKernel panel_kernel(int N);             // negf_panel.cu, up to PNMAX
+constexpr int RNMAX = 72, PNMAX = 272;
 
 struct RgfJob {
     double e_re, e_im;  // complex energy of the solve, E + i*eta already added

@@ -108,3 +108,41 @@ def test_nan_and_singular_blocks_are_reported(oracle):
         D[:, N // 2, 2] = 0.0  # a zero column in the block the right sweep starts from
         _, info = GreensFunction_tri_solver(D, "DF")
         assert info == N // 2 + 1
+
+
+# the panel kernel: panels of 32, row slots of 32 (basis and open channels), at most 320 rows; few jobs, so teams of
+# eight CTAs (up to about 15 jobs), four (33) and two (74)
+@pytest.mark.parametrize("N,nE", [(73, 4), (96, 20), (97, 4), (128, 40), (129, 4), (161, 4), (200, 20), (255, 4),
+                                  (256, 40), (257, 4), (272, 4), (273, 4)])
+def test_panel_teams(oracle, N, nE):
+    args, op, pr = cut_problem(oracle, N, nz=3, grid=64)
+    kin = 0.5 * ((2 * np.pi * pr.nx[:N] / pr.atomic.LX) ** 2 + (2 * np.pi * pr.ny[:N] / pr.atomic.LY) ** 2)
+    # from no open channel to every one (which takes several passes where 2 N > 320)
+    E = np.concatenate([[-1e-6, 1.1 * kin.max() + 1e-5], np.linspace(0.03, 0.6, nE - 2) * kin.max() + 1e-6])
+    ref, _ = oracle.transmission_jobs(op, E, nthreads=8)
+    with Engine(*args) as eng:
+        tau, info = eng.transmission(E)
+        again, _ = eng.transmission(E)
+    assert info == 0
+    np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
+    assert (tau == again).all()
+
+
+def test_panel_batch_of_one_cta_per_job(oracle):
+    """Bases on both sides of 256 in one batch of more jobs than clusters, and a NaN energy among them."""
+    probs = [cut_problem(oracle, N, nz, grid=64) for N, nz in ((180, 3), (260, 2), (75, 5), (263, 3))]
+    E = P.transmission_energies(probs[0][2].atomic, 30)[1:]
+    bad = np.concatenate([E, [np.nan]])
+    engines = [Engine(*p[0]) for p in probs]
+    try:
+        tau, info, stats = transmission_batch(engines, E)
+        tau_bad, info_bad, stats_bad = transmission_batch(engines, bad)
+    finally:
+        for e in engines:
+            e.close()
+    assert info == 0 and stats.n_jobs == len(E) * len(probs)
+    assert info_bad > 0 and stats_bad.n_singular == len(probs)
+    for p, t, b in zip(probs, tau, tau_bad):
+        ref, _ = oracle.transmission_jobs(p[1], E, nthreads=8)
+        np.testing.assert_allclose(t, ref, rtol=RTOL, atol=ATOL)
+        assert (b[:-1] == t).all()
