@@ -34,6 +34,7 @@ constexpr int KC = 16;           // k chunk staged per pipeline step
 // banks, so the four k rows of an m8n8k4 fragment load hit distinct banks.
 constexpr int AP = CM + 2;       // padded row of a k-major A tile
 constexpr int BP = CN + 2;       // padded row of a k-major B tile
+constexpr int TP = 32 + 2;       // padded row of 32 rows of W (trailing_update)
 
 // ------------------------------------------------------------ complex FP64
 __device__ __forceinline__ double2 zmake(double x, double y) { return make_double2(x, y); }
@@ -169,8 +170,8 @@ template <int NB, int RPT>
 __host__ __device__ inline size_t smem_bytes(int N) {
     int ldw = round_up(N, CM);
     size_t big = (size_t)NB * ldw + (size_t)NB * NB;         // sub-panel a + 16x16 block
-    size_t trail = 32 * (size_t)(BP + AP);                    // rank-32 update: gathered rows + W tile
-    if (RPT > 1) trail *= 2;                                  // trailing_update_wide keeps two of each
+    // rank-32 update: gathered rows + 2 x 32 rows of W, or (wide) two of each tile
+    size_t trail = RPT > 1 ? 2 * 32 * (size_t)(BP + AP) : 32 * (size_t)(BP + 2 * TP);
     size_t gemm = 2 * (size_t)KC * (AP + BP);
     if (trail > big) big = trail;
     if (gemm > big) big = gemm;
@@ -503,89 +504,130 @@ __device__ inline double block_sum(double v, const Smem &s) {
 // steps on the other columns, so one pass over the matrix applies KMAX
 // elimination steps.  W tiles are staged from global memory with cp.async;
 // W and the gathered pivot rows feed DMMA warp tiles.
+//
+// Two CTAs share an SM here: 128 registers a thread and 113 KB of shared
+// memory.  The 32 x 64 tiles run rows fastest; while one multiplies, the next
+// one's 32 rows of W arrive by cp.async in the other buffer and its old values
+// in registers, so that only the pivot rows of a new column tile are waited
+// for.
 template <int KMAX>
-__device__ inline void trailing_update(double2 *__restrict__ A, int N, int ld, int k0, int nbt,
-                                       const Smem &s) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm0 = (warp >> 2) * WM, wn0 = (warp & 3) * WN;
+__device__ inline void trailing_update(double2 *__restrict__ A, int N, int ld, int k0, int nbt, const Smem &s) {
+    static_assert(KMAX == 32 && CN == 64 && NT == 256, "4 copies of W and 8 of the pivot rows per thread and tile");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int wm0 = (warp >> 2) * 16, wn0 = (warp & 3) * 16;
     const int nrest = N - nbt;
-    double2 *sB = s.big;               // [KMAX][BP] pivot rows of the column tile
-    double2 *sW = s.big + KMAX * BP;   // [KMAX][AP] rows I0.. of the panel
-    for (int J0 = 0; J0 < nrest; J0 += CN) {
-        // all of a thread's gathers issued before any is stored (loads in flight)
-        {
-            constexpr int Q = (KMAX * CN) / NT;
-            double2 v[Q];
+    double2 *sB = s.big;                // [KMAX][BP] pivot rows of the column tile
+    double2 *sW = s.big + KMAX * BP;    // [2][KMAX][TP] 32 rows of the panel
+    const int nti = (N + 31) / 32, ntj = (nrest + CN - 1) / CN;
+    auto column = [&](int jr) { return A + (size_t)ld * (jr < k0 ? jr : jr + nbt); };
+    auto stage_w = [&](int ti, int bw) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int e = tid + NT * q;
-                const int kk = e / CN, jt = e % CN, jr = J0 + jt;
-                v[q] = make_double2(0.0, 0.0);
-                if (kk < nbt && jr < nrest) {
-                    const int j = jr < k0 ? jr : jr + nbt;
-                    v[q] = A[s.prow[k0 + kk] + (size_t)ld * j];
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int e = tid + NT * q;
-                sB[(e / CN) * BP + e % CN] = v[q];
-            }
+        for (int u = 0; u < 4; ++u) {
+            const int kk = (tid + NT * u) / 32, r = tid % 32, i = ti * 32 + r;
+            const bool v = (kk < nbt) && (i < N);
+            cp_async16(sW + (bw * KMAX + kk) * TP + r, A + (v ? (i + (size_t)ld * (k0 + kk)) : 0), v);
         }
-        int col[2][2];
-        bool cv[2][2];
+    };
+    auto stage_b = [&](int tj) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int kb = tid % KMAX, jt = (tid + NT * u) / KMAX, jr = tj * CN + jt;
+            const bool v = (kb < nbt) && (jr < nrest);
+            cp_async16(sB + kb * BP + jt, v ? column(jr) + s.prow[k0 + kb] : A, v);
+        }
+    };
+    double2 c[2][2][2];
+    auto load = [&](int m, int ti, int tj) {
+        const int i = ti * 32 + wm0 + 8 * m + g;
+        const bool rv = (i < N) && !s.inP[i];
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int jr = J0 + wn0 + 8 * n + 2 * (lane & 3) + e;
-                cv[n][e] = jr < nrest;
-                col[n][e] = jr < k0 ? jr : jr + nbt;
+                const int jr = tj * CN + wn0 + 8 * n + 2 * q + e;
+                c[m][n][e] = make_double2(0.0, 0.0);
+                if (rv && jr < nrest) c[m][n][e] = column(jr)[i];
             }
-        for (int I0 = 0; I0 < N; I0 += CM) {
-#pragma unroll
-            for (int q = 0; q < (KMAX * CM) / NT; ++q) {
-                const int e = tid + NT * q;
-                const int kk = e / CM, r = e % CM, i = I0 + r;
-                const bool v = (kk < nbt) && (i < N);
-                cp_async16(sW + kk * AP + r, A + (v ? (i + (size_t)ld * (k0 + kk)) : 0), v);
-            }
+    };
+    stage_b(0);
+    stage_w(0, 0);
+    cp_async_commit();
+    load(0, 0, 0);
+    load(1, 0, 0);
+    for (int t = 0, ti = 0, tj = 0; t < nti * ntj; ++t) {
+        const int bw = t & 1;
+        int ni = ti + 1, nj = tj;
+        if (ni == nti) { ni = 0; ++nj; }
+        const bool more = nj < ntj, active = (ti * 32 + wm0 < N) && (tj * CN + wn0 < nrest);
+        cp_async_wait<0>();
+        __syncthreads();  // this tile's operands are here; the tile before is done with the other buffer
+        if (more) {
+            stage_w(ni, bw ^ 1);
             cp_async_commit();
-            cp_async_wait<0>();
-            __syncthreads();
-            if ((I0 + wm0 < N) && (J0 + wn0 < nrest)) {
-                WarpAcc acc;
+        }
+        double re[2][2][2], im[2][2][2];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int i = I0 + wm0 + 8 * m + (lane >> 2);
-                    const bool rv = (i < N) && !s.inP[i];
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-                    for (int n = 0; n < 2; ++n)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            double2 c = make_double2(0.0, 0.0);
-                            if (rv && cv[n][e]) c = A[i + (size_t)ld * col[n][e]];
-                            acc.re[m][n][e] = c.x;
-                            acc.im[m][n][e] = c.y;
-                        }
+                for (int e = 0; e < 2; ++e) {
+                    re[m][n][e] = c[m][n][e].x;
+                    im[m][n][e] = c[m][n][e].y;
                 }
-#pragma unroll 2
-                for (int kb = 0; kb < nbt; kb += 4) acc.step(sW, AP, wm0, sB, BP, wn0, kb, lane);
+        const double2 *sa = sW + (bw * KMAX + q) * TP + wm0 + g, *sb = sB + q * BP + wn0 + g;
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int i = I0 + wm0 + 8 * m + (lane >> 2);
-                    if (i < N) {
+        for (int u = 0; u < 8; ++u) {
+            if (more && u < 2) load(u, ni, nj);
+            if (active && 4 * u < nbt) {
+                double2 a[2], b[2];
 #pragma unroll
-                        for (int n = 0; n < 2; ++n)
+                for (int m = 0; m < 2; ++m) a[m] = sa[4 * u * TP + 8 * m];
 #pragma unroll
-                            for (int e = 0; e < 2; ++e)
-                                if (cv[n][e]) A[i + (size_t)ld * col[n][e]] = make_double2(acc.re[m][n][e], acc.im[m][n][e]);
+                for (int n = 0; n < 2; ++n) b[n] = sb[4 * u * BP + 8 * n];
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        dmma(re[m][n][0], re[m][n][1], a[m].x, b[n].x);
+                        dmma(im[m][n][0], im[m][n][1], a[m].x, b[n].y);
+                    }
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const double na = -a[m].y;
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        dmma(re[m][n][0], re[m][n][1], na, b[n].y);
+                        dmma(im[m][n][0], im[m][n][1], a[m].y, b[n].x);
                     }
                 }
             }
-            __syncthreads();
         }
+        if (active) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int jr = tj * CN + wn0 + 8 * n + 2 * q + e;
+                    if (jr < nrest) {
+                        double2 *col = column(jr);
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+                            const int i = ti * 32 + wm0 + 8 * m + g;
+                            if (i < N) col[i] = make_double2(re[m][n][e], im[m][n][e]);
+                        }
+                    }
+                }
+        }
+        if (nj != tj && more) {
+            __syncthreads();  // the column tile's pivot rows are read
+            stage_b(nj);
+            cp_async_commit();
+        }
+        ti = ni;
+        tj = nj;
     }
+    __syncthreads();
 }
 
 // The same update for the variants of one CTA per SM (RPT > 1), where nothing
