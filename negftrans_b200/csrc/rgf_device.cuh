@@ -129,21 +129,15 @@ struct Geo {
     int lead_model;         // 0 reference continuum lead term, 1 exact lattice surface GF
 };
 
-// One warp's pivot candidate: a sortable key and the reciprocal of its value.
+// The warps' pivot candidates of one step.  A key is the high word of
+// |re|+|im| (non-negative doubles order as integers) with the warp in its low
+// bits: one integer reduction inside a warp, one comparison over the warps,
+// and two magnitudes that agree to 17 bits count as a tie.  -1 = no candidate,
+// below 8 = a zero pivot.
 struct Red {
-    unsigned long long key;
-    unsigned long long pad;
-    double2 d;
+    double2 d[NWARP];   // the reciprocals of the candidates
+    int key[NWARP], row[NWARP];
 };
-
-// Key that orders candidates by |re|+|im| (v >= 0, so its bit pattern sorts
-// as an unsigned integer), then by lower row index.  The low 11 bits of v
-// carry the index; two magnitudes that agree in all but those bits (a
-// relative difference below 2^-41) count as a tie.  Key 0 = no candidate.
-__device__ __forceinline__ unsigned long long pivot_key(double v, int row) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    return (b & ~0x7FFull) | (unsigned long long)(0x7FF - row);
-}
 
 // Shared memory carve-up (dynamic).
 struct Smem {
@@ -158,7 +152,7 @@ struct Smem {
     double *gL;     // [N] gamma_L  sin(q dz)/dz^2 (grid.f90:365)
     double *gR;     // [N] gamma_R
     double2 *cand;  // [2][NWARP][32] each warp's pivot candidate row (double-buffered by step)
-    Red *red;       // [2][NWARP] each warp's candidate key and reciprocal
+    Red *red;       // [2] the warps' candidates, by the step's parity
     double *fred;   // [NWARP] float reductions
     double2 *big;   // union: sub-panel + block | trailing rows + W tile | GEMM stages
     int ldw;
@@ -180,7 +174,7 @@ __host__ __device__ inline size_t smem_bytes(int N) {
     b += 2 * (size_t)round_up(N, 2) * sizeof(double2);
     b += 2 * (size_t)round_up(N, 2) * sizeof(double);
     b += 2 * NWARP * 32 * sizeof(double2);
-    b += 2 * NWARP * sizeof(Red) + NWARP * sizeof(double);
+    b += 2 * sizeof(Red) + NWARP * sizeof(double);
     b = (b + 255) / 256 * 256;
     return b + big * sizeof(double2);
 }
@@ -202,7 +196,7 @@ __device__ inline Smem carve(unsigned char *base, int N) {
     s.gR = s.gL + n2;
     s.cand = (double2 *)(s.gR + n2);
     s.red = (Red *)(s.cand + 2 * NWARP * 32);
-    s.fred = (double *)(s.red + 2 * NWARP);
+    s.fred = (double *)(s.red + 2);
     size_t off = (size_t)((unsigned char *)(s.fred + NWARP) - base);
     off = (off + 255) / 256 * 256;
     s.big = (double2 *)(base + off);
@@ -728,48 +722,42 @@ __device__ inline void trailing_update_wide(double2 *__restrict__ A, int N, int 
     __syncthreads();
 }
 
-// Gauss-Jordan elimination of the columns [kb, kb+nbe) of a register panel
-// w (row tid + NT*r of the block in w[r][.]), with implicit partial pivoting:
-// the pivot of each column is the unused row with the largest |re|+|im|
-// (lowest index on ties), as zgetf2 chooses.  Pivot rows get inP = tag.
-// The step loop is not unrolled: columns are picked out of the register rows
-// by predication, which keeps the code size O(NB).  Each step updates the
-// next pivot column first and runs its warp-level argmax while the rest of
-// the row is updated; the winning lane of each warp computes the reciprocal
-// of its candidate before the barrier.
 // Warp-level pivot candidate for the column values f: writes the warp's best
-// key and the reciprocal of its value into red[buf][warp]; returns, in the
+// key, its row and the reciprocal of its value into red[buf]; returns, in the
 // winning thread, the register row r of the candidate (-1 elsewhere).  That
 // thread publishes the candidate's updated row into cand[buf][warp] later.
+// Every lane takes the reciprocal of its own best value while the reduction
+// runs (1 / 1 where it has none: a division by zero would take the slow path).
 template <int NB, int RPT>
 __device__ inline int warp_pivot(const double2 (&f)[RPT], unsigned used, int buf, const Smem &s) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned long long key = 0;
-    int rbest = -1;
+    int key = -1, rbest = -1;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
         if (!((used >> r) & 1u)) {
-            double v = cabs1(f[r]);
-            if (!(v == v)) v = 0.0;  // NaN rows rank as zero pivots
-            const unsigned long long k = pivot_key(v, tid + NT * r);
+            int k = __double2hiint(cabs1(f[r]));
+            if ((unsigned)k >= 0x7ff80000u) k = 0;  // a NaN ranks as a zero pivot
+            k = (k & ~7) | warp;
             if (k > key) { key = k; rbest = r; }
         }
     }
-    unsigned long long wk = key;
+    double2 best = make_double2(1.0, 0.0);
+    const unsigned hot = key < 8 ? 0u : 1u << rbest;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, wk, o);
-        wk = ok > wk ? ok : wk;
+    for (int r = 0; r < RPT; ++r) {
+        const bool mine = (hot >> r) & 1u;  // as a bit: equality with r is turned into an indexed load
+        best.x = mine ? f[r].x : best.x;
+        best.y = mine ? f[r].y : best.y;
     }
-    Red *red = s.red + buf * NWARP;
-    if (lane == 0) red[warp].key = wk;
-    if (wk != 0 && key == wk) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r)
-            if (r == rbest) red[warp].d = zrcp(f[r]);
-        return rbest;
-    }
-    return -1;
+    const int top = __reduce_max_sync(0xffffffffu, key);
+    double2 d = zrcp(best);
+    if (lane != __ffs(__ballot_sync(0xffffffffu, key == top)) - 1) return -1;
+    if (key >= 0 && key < 8) d = zrcp(make_double2(0.0, 0.0));  // a zero pivot: the job is reported
+    Red &red = s.red[buf];
+    red.d[warp] = d;
+    red.key[warp] = key;
+    red.row[warp] = tid + NT * rbest;
+    return rbest;
 }
 
 // Gauss-Jordan elimination of the columns [kb, kb+nbe) of a register panel w
@@ -802,18 +790,13 @@ __device__ inline void factor_subpanel(double2 (&w)[RPT][NB], int kb, int nbe, u
         if (kk < nbe) {
             const int buf = kk & 1;
             __syncthreads();
-            const Red *red = s.red + buf * NWARP;
-            unsigned long long key = red[0].key;
-            int q = 0;
-#pragma unroll
-            for (int j = 1; j < NWARP; ++j) {
-                const unsigned long long k = red[j].key;
-                if (k > key) { key = k; q = j; }
-            }
-            const double2 d = red[q].d;
+            const Red &red = s.red[buf];
+            const int4 ka = *(const int4 *)red.key, kc = *(const int4 *)(red.key + 4);
+            const int top = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kc.x, kc.y), max(kc.z, kc.w)));
+            const int q = top & 7, p = red.row[q];
+            const double2 d = red.d[q];
             const double2 *srow = s.cand + (buf * NWARP + q) * 32;
-            const int p = 0x7FF - (int)(key & 0x7FFull);
-            if ((key >> 11) == 0 && info == 0) info = kb + kk + 1;
+            if (top < 8 && info == 0) info = kb + kk + 1;
 #pragma unroll
             for (int r = 0; r < RPT; ++r)
                 if (tid + NT * r == p) used |= 1u << r;
