@@ -456,14 +456,30 @@ int slab_jobs_in_flight(negf_ctx *c, size_t per_job_bytes, int njobs) {
     return std::max(b, 0);
 }
 
+// A caller's output buffer, to be made resident while the GPU works.  The pages
+// of a fresh buffer (NumPy's zeros, a first malloc) are mapped at their first
+// touch, which costs more than the copy into them: 62 MB to the host 29 ms into
+// fresh pages, 3.7 ms into touched ones.  Contents stay as they are.
+struct HostOut {
+    void *p = nullptr;
+    size_t bytes = 0;
+    void touch() {
+        volatile char *c = (volatile char *)p;
+        for (size_t i = 0; i < bytes; i += 4096) c[i] = c[i];
+        if (bytes) c[bytes - 1] = c[bytes - 1];
+        bytes = 0;
+    }
+};
+
 // Runs the D-mode sweeps for `jobs` in chunks and forms the weighted sums of
 // their diagonal blocks, 2 dz^2 G_kk scaled by coef[job]:
 //   gsz == 0: every job sums into out[0] (density; chunks accumulate);
 //   gsz  > 0: jobs [o*gsz, (o+1)*gsz) sum into out[o] (LDOS per energy).
 // want selects the slab mode (WANT_D, or WANT_D | WANT_A [| WANT_MIRROR] with
 // the per-job cd / ca).
+// out: the host buffer that d_out will be copied to (touched during the first chunk).
 int diag_accumulate(negf_ctx *c, const std::vector<RgfJob> &jobs, const std::vector<double2> &coef,
-                    int gsz, double2 *d_out, std::vector<int> &info_all, double &ms_total,
+                    int gsz, double2 *d_out, std::vector<int> &info_all, double &ms_total, HostOut out,
                     int want = WANT_D) {
     const int njobs = (int)jobs.size();
     const int N = c->N, Nz = c->Nz, ld = c->ld;
@@ -502,8 +518,9 @@ int diag_accumulate(negf_ctx *c, const std::vector<RgfJob> &jobs, const std::vec
         k_accumulate<<<blocks, 256, 0, c->stream>>>(d_slabs, sstride, ld, N, Nz, d_coef, gs, nout,
                                                     c->Lz / Nz, acc, d_out + (size_t)o0 * N * N * Nz);
         float ms = 0.f;
-        if (cudaGetLastError() || cudaEventRecord(c->ev1, c->stream) ||
-            cudaMemcpyAsync(info_all.data() + j0, d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream) ||
+        if (cudaGetLastError() || cudaEventRecord(c->ev1, c->stream)) { rc = NEGF_ERR_CUDA; break; }
+        out.touch();
+        if (cudaMemcpyAsync(info_all.data() + j0, d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream) ||
             cudaStreamSynchronize(c->stream) || cudaEventElapsedTime(&ms, c->ev0, c->ev1)) {
             rc = NEGF_ERR_CUDA;
             break;
@@ -733,10 +750,14 @@ int negf_autotune(negf_ctx *c, const double *energies, int32_t nE, int32_t *chos
     return bv >= 0 ? NEGF_OK : NEGF_ERR_UNSUPPORTED;
 }
 
-int negf_density(negf_ctx *c, int32_t n_circle, int32_t n_line, double min_v, double mu, double gap,
-                 double temperature, double *dm, negf_stats *stats) {
-    if (!c || !dm || n_circle < 2 || n_line < 2) return NEGF_ERR_ARG;
-    if (cudaSetDevice(c->device) != cudaSuccess) return NEGF_ERR_CUDA;
+}  // extern "C"
+
+namespace {
+// Density_Matrix of the reference's contour on the device: *d_out (freed by the
+// caller) holds N x N x Nz.  dm, if any, is the host buffer it will go to.
+int density_device(negf_ctx *c, int32_t n_circle, int32_t n_line, double min_v, double mu, double gap, double temperature,
+                   HostOut dm, double2 **d_out, std::vector<int> &info, double &ms) {
+    *d_out = nullptr;
     // contour of negf.f90:37-65 and weights of negf.f90:86-111
     const double circle_L = min_v - 1.0 / HARTREE, circle_R = mu - gap;
     const double line_L = mu - gap, line_R = mu + gap;
@@ -783,15 +804,23 @@ int negf_density(negf_ctx *c, int32_t n_circle, int32_t n_line, double min_v, do
         coef[job] = cf;
     }
     const size_t per = (size_t)c->N * c->N * c->Nz;
+    if (cudaMalloc(d_out, sizeof(double2) * per) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
+    return diag_accumulate(c, jobs, coef, 0, *d_out, info, ms, dm);
+}
+}  // namespace
+
+extern "C" {
+
+int negf_density(negf_ctx *c, int32_t n_circle, int32_t n_line, double min_v, double mu, double gap,
+                 double temperature, double *dm, negf_stats *stats) {
+    if (!c || !dm || n_circle < 2 || n_line < 2) return NEGF_ERR_ARG;
+    if (cudaSetDevice(c->device) != cudaSuccess) return NEGF_ERR_CUDA;
+    const size_t bytes = sizeof(double2) * (size_t)c->N * c->N * c->Nz;
     double2 *d_out = nullptr;
-    if (cudaMalloc(&d_out, sizeof(double2) * per) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
     std::vector<int> info;
     double ms = 0;
-    int rc = diag_accumulate(c, jobs, coef, 0, d_out, info, ms);
-    if (!rc) {
-        cudaError_t e = cudaMemcpy(dm, d_out, sizeof(double2) * per, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) rc = NEGF_ERR_CUDA;
-    }
+    int rc = density_device(c, n_circle, n_line, min_v, mu, gap, temperature, HostOut{dm, bytes}, &d_out, info, ms);
+    if (!rc && cudaMemcpy(dm, d_out, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) rc = NEGF_ERR_CUDA;
     cudaFree(d_out);
     if (rc) return rc;
     fill_stats(stats, info, ms);
@@ -822,7 +851,7 @@ int negf_density_accumulate(negf_ctx *c, const double *energies, const double *w
     if (cudaMalloc(&d_out, sizeof(double2) * per) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
     std::vector<int> info;
     double ms = 0;
-    int rc = diag_accumulate(c, jobs, coef, 0, d_out, info, ms);
+    int rc = diag_accumulate(c, jobs, coef, 0, d_out, info, ms, HostOut{dm, sizeof(double2) * per});
     if (!rc && cudaMemcpy(dm, d_out, sizeof(double2) * per, cudaMemcpyDeviceToHost) != cudaSuccess) rc = NEGF_ERR_CUDA;
     cudaFree(d_out);
     if (rc) return rc;
@@ -887,7 +916,7 @@ int negf_density_neq(negf_ctx *c, int32_t n_circle, int32_t n_window, double min
     if (cudaMalloc(&d_out, sizeof(double2) * per) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
     std::vector<int> info;
     double ms = 0;
-    int rc = diag_accumulate(c, jobs, unit, 0, d_out, info, ms,
+    int rc = diag_accumulate(c, jobs, unit, 0, d_out, info, ms, HostOut{dm, sizeof(double2) * per},
                              WANT_D | WANT_A | (right_injects ? WANT_MIRROR : 0));
     if (!rc && cudaMemcpy(dm, d_out, sizeof(double2) * per, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = NEGF_ERR_CUDA;
@@ -920,7 +949,7 @@ int negf_ldos_matrix(negf_ctx *c, double e_lo, double e_hi, int32_t n_e, int32_t
     if (cudaMalloc(&d_out, sizeof(double2) * per * n_chunk) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
     std::vector<int> info;
     double ms = 0;
-    int rc = diag_accumulate(c, jobs, coef, nk, d_out, info, ms);
+    int rc = diag_accumulate(c, jobs, coef, nk, d_out, info, ms, HostOut{ldos, sizeof(double2) * per * n_chunk});
     if (!rc && cudaMemcpy(ldos, d_out, sizeof(double2) * per * n_chunk, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = NEGF_ERR_CUDA;
     cudaFree(d_out);
@@ -941,78 +970,89 @@ int negf_tri_solve(negf_ctx *ctx, const double *D, int32_t N, int32_t Nz, const 
     if (strpbrk(dfl, "Ll")) want |= WANT_L;
     const size_t per = (size_t)N * N * Nz;
     const size_t bytes = sizeof(double2) * per;
-    // the reference zero-fills every plane (math_kernel.f90:75-77)
-    if (diag) memset(diag, 0, bytes);
-    if (first) memset(first, 0, bytes);
-    if (last) memset(last, 0, bytes);
-    negf_ctx local;
-    negf_ctx *c = &local;
-    c->device = dev;
-    cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
+    // Pass 0: generator_r sweep, diagonal and first-column blocks; pass 1:
+    // generator_l sweep and last-column blocks, beside it with a slab of its own.
+    negf_ctx local[2];
+    const int wants[2] = {want & ((diag ? WANT_D : 0) | (first ? WANT_F : 0)), want & (last ? WANT_L : 0)};
+    double *outs[2] = {first, last};
+    double2 *d_D = nullptr, *d_slab[2] = {}, *d_out[2] = {};
+    int *d_nx = nullptr, *d_info = nullptr;
+    RgfJob *d_job = nullptr;
+    int rc = 0, hinfo[2] = {0, 0};
     Geo g{};
     g.N = N; g.Nz = Nz; g.ld = round_up(N, 8);
     g.delta = 1.0; g.c2 = 1.0;
     g.lead_model = 0;
-    double2 *d_D = nullptr, *d_slab = nullptr, *d_first = nullptr, *d_last = nullptr;
-    int *d_nx = nullptr, *d_ny = nullptr, *d_info = nullptr;
-    int rc = 0, hinfo = 0;
     const size_t sstride = (size_t)g.ld * N * Nz;
-    cudaStream_t st = nullptr;
-#define CKT(x) do { if ((x) != cudaSuccess) { rc = NEGF_ERR_CUDA; goto done; } } while (0)
-    CKT(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    CKT(cudaMalloc(&d_D, bytes));
-    CKT(cudaMalloc(&d_slab, sizeof(double2) * sstride));
-    CKT(cudaMalloc(&d_nx, sizeof(int) * N));
-    CKT(cudaMalloc(&d_ny, sizeof(int) * N));
-    CKT(cudaMalloc(&d_info, sizeof(int)));
-    CKT(cudaMemset(d_nx, 0, sizeof(int) * N));
-    CKT(cudaMemset(d_ny, 0, sizeof(int) * N));
-    if ((want & WANT_F) && first) CKT(cudaMalloc(&d_first, bytes));
-    if ((want & WANT_L) && last) CKT(cudaMalloc(&d_last, bytes));
-    CKT(cudaMemcpy(d_D, D, bytes, cudaMemcpyHostToDevice));
-    g.nx = d_nx; g.ny = d_ny;
-    {
-        RgfJob jb{};
-        RgfJob *d_job = nullptr;
-        int i2 = 0;
-        CKT(cudaMalloc(&d_job, sizeof(RgfJob)));
-        CKT(cudaMemcpy(d_job, &jb, sizeof(RgfJob), cudaMemcpyHostToDevice));
-        // pass 1: generator_r sweep, diagonal and first-column blocks
-        int w = want & (WANT_D | WANT_F);
-        if (!diag) w &= ~WANT_D;
-        if (!first) w &= ~WANT_F;
-        if (w) {
-            rc = slab_launch(c, g, d_job, 1, d_D, d_slab, sstride, w, d_first, nullptr, d_info, st);
-            if (!rc && (cudaStreamSynchronize(st) != cudaSuccess ||
-                        cudaMemcpy(&hinfo, d_info, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess))
-                rc = NEGF_ERR_CUDA;
-            if (!rc && (w & WANT_D) &&
-                cudaMemcpy2D(diag, sizeof(double2) * N, d_slab, sizeof(double2) * g.ld, sizeof(double2) * N,
-                             (size_t)N * Nz, cudaMemcpyDeviceToHost) != cudaSuccess)
-                rc = NEGF_ERR_CUDA;
-        }
-        // pass 2: generator_l sweep and last-column blocks (reuses the slab)
-        if (!rc && (want & WANT_L) && last) {
-            rc = slab_launch(c, g, d_job, 1, d_D, d_slab, sstride, WANT_L, nullptr, d_last, d_info, st);
-            if (!rc && (cudaStreamSynchronize(st) != cudaSuccess ||
-                        cudaMemcpy(&i2, d_info, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess))
-                rc = NEGF_ERR_CUDA;
-            if (!hinfo) hinfo = i2;
-        }
-        cudaFree(d_job);
-        if (rc) goto done;
+#define CKT(x) do { if ((x) != cudaSuccess) { cudaGetLastError(); rc = NEGF_ERR_CUDA; goto done; } } while (0)
+    for (negf_ctx &c : local) {
+        c.device = dev;
+        cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, dev);
+        CKT(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     }
-    if (d_first) CKT(cudaMemcpy(first, d_first, bytes, cudaMemcpyDeviceToHost));
-    if (d_last) CKT(cudaMemcpy(last, d_last, bytes, cudaMemcpyDeviceToHost));
+    CKT(cudaMalloc(&d_D, bytes));
+    CKT(cudaMalloc(&d_nx, sizeof(int) * N));
+    CKT(cudaMalloc(&d_info, 2 * sizeof(int)));
+    CKT(cudaMalloc(&d_job, sizeof(RgfJob)));
+    CKT(cudaMemset(d_nx, 0, sizeof(int) * N));
+    CKT(cudaMemset(d_job, 0, sizeof(RgfJob)));
+    CKT(cudaMemcpy(d_D, D, bytes, cudaMemcpyHostToDevice));
+    g.nx = g.ny = d_nx;
+    {
+        auto launch = [&](int p, double2 *slab) {
+            return slab_launch(&local[p], g, d_job, 1, d_D, slab, sstride, wants[p], p == 0 ? d_out[0] : nullptr,
+                               p == 1 ? d_out[1] : nullptr, d_info + p, local[p].stream);
+        };
+        // waits for pass p and copies its planes out of slab and d_out[p]
+        auto collect = [&](int p, const double2 *slab) {
+            if (cudaStreamSynchronize(local[p].stream) != cudaSuccess ||
+                cudaMemcpy(&hinfo[p], d_info + p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+                return NEGF_ERR_CUDA;
+            if ((wants[p] & WANT_D) && cudaMemcpy2D(diag, sizeof(double2) * N, slab, sizeof(double2) * g.ld, sizeof(double2) * N,
+                                                   (size_t)N * Nz, cudaMemcpyDeviceToHost) != cudaSuccess)
+                return NEGF_ERR_CUDA;
+            if (d_out[p] && cudaMemcpy(outs[p], d_out[p], bytes, cudaMemcpyDeviceToHost) != cudaSuccess) return NEGF_ERR_CUDA;
+            return 0;
+        };
+        bool pending[2] = {false, false};
+        for (int p = 0; p < 2; ++p)
+            if (wants[p] & (WANT_F | WANT_L)) CKT(cudaMalloc(&d_out[p], bytes));
+        for (int p = 0; p < 2 && !rc; ++p) {
+            if (!wants[p]) continue;
+            if (cudaMalloc(&d_slab[p], sizeof(double2) * sstride) != cudaSuccess) {
+                cudaGetLastError();
+                if (!pending[0]) { rc = NEGF_ERR_CUDA; break; }
+                break;  // no room for a second slab: the passes one after the other, below
+            }
+            rc = launch(p, d_slab[p]);
+            pending[p] = !rc;
+        }
+        // the reference zero-fills every plane (math_kernel.f90:75-77); this also
+        // maps its pages while the GPU works
+        if (diag) memset(diag, 0, bytes);
+        if (first) memset(first, 0, bytes);
+        if (last) memset(last, 0, bytes);
+        if (!rc && pending[0]) rc = collect(0, d_slab[0]);
+        if (!rc && wants[1] && !pending[1]) {
+            rc = launch(1, d_slab[0]);
+            pending[1] = !rc;
+        }
+        if (!rc && pending[1]) rc = collect(1, nullptr);
+    }
 #undef CKT
 done:
-    cudaFree(d_D); cudaFree(d_slab); cudaFree(d_first); cudaFree(d_last);
-    cudaFree(d_nx); cudaFree(d_ny); cudaFree(d_info);
-    cudaFree(c->d_ws);
-    c->d_ws = nullptr;
-    if (st) cudaStreamDestroy(st);
+    for (int p = 0; p < 2; ++p) {
+        if (local[p].stream) {
+            cudaStreamSynchronize(local[p].stream);
+            cudaStreamDestroy(local[p].stream);
+        }
+        cudaFree(d_slab[p]);
+        cudaFree(d_out[p]);
+        cudaFree(local[p].d_ws);
+    }
+    cudaFree(d_D); cudaFree(d_nx); cudaFree(d_info); cudaFree(d_job);
     if (rc) return rc;
-    return hinfo;
+    return hinfo[0] ? hinfo[0] : hinfo[1];
 }
 
 }  // extern "C"
@@ -1228,27 +1268,28 @@ extern "C" int negf_density_real(negf_ctx *c, int32_t n_circle, int32_t n_line, 
                                  double gap, double temperature, int32_t Nx, int32_t Ny, double scale,
                                  double *density, double *dm, negf_stats *stats) {
     if (!c || !density || Nx < 1 || Ny < 1) return NEGF_ERR_ARG;
-    const size_t per = (size_t)c->N * c->N * c->Nz;
-    std::vector<double> host_dm;
-    double *dmh = dm;
-    if (!dmh) { host_dm.resize(2 * per); dmh = host_dm.data(); }
-    int rc = negf_density(c, n_circle, n_line, min_v, mu, gap, temperature, dmh, stats);
-    if (rc < 0) return rc;
-    const int info = rc;
+    if (n_circle < 2 || n_line < 2) return NEGF_ERR_ARG;
+    if (cudaSetDevice(c->device) != cudaSuccess) return NEGF_ERR_CUDA;
+    const size_t per = (size_t)c->N * c->N * c->Nz, nd = (size_t)Nx * Ny * c->Nz;
     double2 *d_G = nullptr;
     double *d_dens = nullptr;
-    const size_t nd = (size_t)Nx * Ny * c->Nz;
-    if (cudaMalloc(&d_G, sizeof(double2) * per) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
-    if (cudaMalloc(&d_dens, sizeof(double) * nd) != cudaSuccess) { cudaGetLastError(); cudaFree(d_G); return NEGF_ERR_NOMEM; }
-    rc = 0;
-    if (cudaMemcpyAsync(d_G, dmh, sizeof(double2) * per, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) rc = NEGF_ERR_CUDA;
+    std::vector<int> info;
+    double ms = 0;
+    int rc = density_device(c, n_circle, n_line, min_v, mu, gap, temperature,
+                            dm ? HostOut{dm, sizeof(double2) * per} : HostOut{density, sizeof(double) * nd}, &d_G, info, ms);
+    // the matrix goes to the host before the real-space step, which may refuse the grid
+    if (!rc) {
+        fill_stats(stats, info, ms);
+        if (dm && cudaMemcpy(dm, d_G, sizeof(double2) * per, cudaMemcpyDeviceToHost) != cudaSuccess) rc = NEGF_ERR_CUDA;
+    }
+    if (!rc && cudaMalloc(&d_dens, sizeof(double) * nd) != cudaSuccess) { cudaGetLastError(); rc = NEGF_ERR_NOMEM; }
     if (!rc) rc = launch_ptor(c, d_G, c->Nz, Nx, Ny, scale, d_dens, nullptr, c->stream);
     if (!rc && (cudaMemcpyAsync(density, d_dens, sizeof(double) * nd, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
                 cudaStreamSynchronize(c->stream) != cudaSuccess))
         rc = NEGF_ERR_CUDA;
     cudaFree(d_G);
     cudaFree(d_dens);
-    return rc ? rc : info;
+    return rc ? rc : first_info(info);
 }
 
 extern "C" int negf_vhat_gpu(const double *vreal, int32_t Nx, int32_t Ny, int32_t Nz, int32_t ngx, int32_t ngy,
@@ -1347,6 +1388,7 @@ int ldos_one_kpoint(negf_ctx *c, double e_lo, double e_hi, int n_e, const int32_
     const double f = -(c->kpt[2] / PI) * 2.0 * (c->Lz / Nz) * (c->Lz / Nz);  // negf.f90:230-231, :78
     std::vector<int> info_all(n_e, 0);
     double ms_all = 0;
+    HostOut out{ldos, sizeof(double) * nout * n_e};
     Geo g = make_geo(c);
     if (!rc && cudaMemsetAsync(d_out, 0, sizeof(double) * nout * n_e, c->stream) != cudaSuccess) rc = NEGF_ERR_CUDA;
     for (int e0 = 0; e0 < n_e && !rc; e0 += b) {
@@ -1363,8 +1405,9 @@ int ldos_one_kpoint(negf_ctx *c, double e_lo, double e_hi, int n_e, const int32_
         if ((rc = slab_launch(c, g, d_jobs, nb, nullptr, d_slabs, sstride, WANT_D, nullptr, nullptr, d_info, c->stream)))
             break;
         float ms = 0.f;
-        if (cudaEventRecord(c->ev1, c->stream) ||
-            cudaMemcpyAsync(info_all.data() + e0, d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream)) {
+        if (cudaEventRecord(c->ev1, c->stream)) { rc = NEGF_ERR_CUDA; break; }
+        out.touch();
+        if (cudaMemcpyAsync(info_all.data() + e0, d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream)) {
             rc = NEGF_ERR_CUDA;
             break;
         }
@@ -1419,6 +1462,7 @@ extern "C" int negf_ldos(negf_ctx *c, double e_lo, double e_hi, int32_t n_e, con
     int rc = cudaMemsetAsync(d_out, 0, sizeof(double) * nout * n_e, c->stream) == cudaSuccess ? 0 : NEGF_ERR_CUDA;
     std::vector<int> info_all;
     double ms_all = 0;
+    HostOut out{ldos, sizeof(double) * nout * n_e};
     for (int e0 = 0; e0 < n_e && !rc; e0 += chunk) {
         const int nc = std::min(chunk, n_e - e0);
         std::vector<RgfJob> jobs(nc * nk);
@@ -1435,7 +1479,8 @@ extern "C" int negf_ldos(negf_ctx *c, double e_lo, double e_hi, int32_t n_e, con
         }
         std::vector<int> info;
         double ms = 0;
-        rc = diag_accumulate(c, jobs, coef, nk, d_mat, info, ms);
+        rc = diag_accumulate(c, jobs, coef, nk, d_mat, info, ms, out);
+        out.bytes = 0;
         if (rc) break;
         info_all.insert(info_all.end(), info.begin(), info.end());
         ms_all += ms;
