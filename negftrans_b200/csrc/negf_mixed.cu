@@ -1905,6 +1905,9 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pass(MixedArgs a, int mode, int
     if (cpj > 1) cluster_sync();
 }
 
+template <int MT>
+struct Tiles { static constexpr int v = MT; };
+
 // FP64 residual of the block-tridiagonal system for x0, one CTA per (job,
 // slice b): r(b) = E_1 delta_b0 - x0(b-1) - D_b x0(b) - x0(b+1), D_b in FP64
 // and the product on the FP64 tensor cores (DMMA warp tiles of
@@ -1944,13 +1947,14 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_residual(MixedArgs a) {
     float2 *out = (float2 *)(jm + L.off_rc) + b * sl;
     const double2 *vs = g.vhat + (size_t)g.W * g.H * b;
     const double2 *vt = a.voff + (size_t)N * L.ld * b;
-    const int wm0 = (warp >> 2) * negf::WM, wn0 = (warp & 3) * negf::WN;
     const int nkc = (N + KC - 1) / KC;
     constexpr int BQ = (KC * CN) / NT;  // x0 values per thread per chunk
-    for (int J0 = 0; J0 < npad; J0 += CN) {
+    // 64 rows x 64 columns J0.. : warp tiles of MT m8 tiles x 16 columns at (wm0, wn0)
+    auto columns = [&](auto mt, int J0, int wm0, int wn0) {
+        constexpr int MT = decltype(mt)::v;
         for (int I0 = 0; I0 < N; I0 += CM) {
             const bool active = (I0 + wm0 < N) && (J0 + wn0 < npad);
-            negf::WarpAcc acc;
+            negf::WarpTile<MT> acc;
             acc.zero();
             float2 xr[BQ];
             auto load_a = [&](int st, int k0) {
@@ -2002,7 +2006,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_residual(MixedArgs a) {
             __syncthreads();
             if (active) {
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < MT; ++m) {
                     const int i = I0 + wm0 + 8 * m + (lane >> 2);
                     double2 dfix = make_double2(0.0, 0.0);
                     if (i < N) {
@@ -2033,6 +2037,14 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_residual(MixedArgs a) {
                 }
             }
         }
+    };
+    // Warp w issues on sub-partition w % 4.  With more than 32 columns left the
+    // four column strips of 32 x 16 warp tiles keep the four of them busy; with
+    // 32 or fewer, half or more of those strips would be empty, so the four
+    // sub-partitions take 16 rows each instead.
+    for (int J0 = 0; J0 < npad; J0 += CN) {
+        if (npad - J0 > 32) columns(Tiles<4>(), J0, (warp >> 2) * negf::WM, (warp & 3) * negf::WN);
+        else columns(Tiles<2>(), J0, (warp & 3) * 16, (warp >> 2) * negf::WN);
     }
 }
 

@@ -331,12 +331,13 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// Complex accumulators of one warp tile: 4 x 2 m8n8 tiles, 2 elements each.
-struct WarpAcc {
-    double re[4][2][2], im[4][2][2];
+// Complex accumulators of one warp tile: MT x 2 m8n8 tiles, 2 elements each.
+template <int MT>
+struct WarpTile {
+    double re[MT][2][2], im[MT][2][2];
     __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -346,23 +347,23 @@ struct WarpAcc {
     __device__ __forceinline__ void step(const double2 *sA, int lda, int arow, const double2 *sB, int ldb,
                                          int bcol, int kb, int lane) {
         const int kk = kb + (lane & 3), g = lane >> 2;
-        double2 a[4], b[2];
+        double2 a[MT], b[2];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) a[m] = sA[kk * lda + arow + 8 * m + g];
+        for (int m = 0; m < MT; ++m) a[m] = sA[kk * lda + arow + 8 * m + g];
 #pragma unroll
         for (int n = 0; n < 2; ++n) b[n] = sB[kk * ldb + bcol + 8 * n + g];
 #pragma unroll
         // first the a.re products of all tiles, then the a.im ones, so that
         // the two MMAs into one accumulator are 16 instructions apart
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
                 dmma(re[m][n][0], re[m][n][1], a[m].x, b[n].x);
                 dmma(im[m][n][0], im[m][n][1], a[m].x, b[n].y);
             }
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < MT; ++m) {
             const double nai = -a[m].y;
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
@@ -372,6 +373,7 @@ struct WarpAcc {
         }
     }
 };
+using WarpAcc = WarpTile<4>;
 
 // C(i,j) = sum_k A(i, acol[k]) * B(k, bcol[j]) for one CTA, complex FP64.
 // acol/bcol == nullptr means identity.  Modes of the epilogue:
