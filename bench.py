@@ -388,7 +388,8 @@ def run_ours_fp64(args):
             "vs_baseline": None, "dtype": "c128", "data": "synthetic",
             "config": workload_config(args.workload, N, Nz, w.n_energy, nk),
             "step": {"energies_per_gpu": B, "precision": "fp64", "parallelism": f"energy-sharded x{world}",
-                     "l2": "256 MB buffer written between timed steps; per-job workspace "
+                     "l2": "256 MB buffer written between timed steps" if N <= 72 else
+                           "256 MB buffer written between timed steps; workspace "
                            f"{4 * ((N + 7) // 8 * 8) * N * 16 * min(B * nk, 148) / 1e6:.0f} MB > L2"},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
@@ -400,7 +401,8 @@ def run_ours_fp64(args):
                          "peak_source": "measured in-run: cuBLAS FP64 GEMM 8192^3 (MEASURED_PEAKS.json "
                                         "has no FP64 figure)",
                          "flops_per_launch": fl,
-                         "kernel": ("k_transmission<8,1,2>" if N <= 256 else
+                         "kernel": ("k_register" if N <= 72 else "k_transmission<8,1,2>" if N <= 256 else
+                                    "k_panel" if N <= 272 else
                                     "k_transmission<16,2,1>" if N <= 512 else "k_transmission<8,4,1>"),
                          "flops_note": "executed: 8N^3 per inverse + 8 n_open N^2 per chain product "
                                        "(rows of G_{Nz,1} with gamma_L != 0); the reference's "

@@ -34,8 +34,8 @@ enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, VCHIP = 3, VNONE = 4 };
 // few (at most one per two SMs: nine jobs of N = 221, N_z = 160, 175 -> 86 ms in
 // teams of eight) or N > 256 (the next variant takes a whole SM as
 // well, at two rows per thread); otherwise 8 x 1 x 2, whose two jobs per SM
-// cover each other's pivots (N = 221: 920 us of an SM per slice and job, the
-// panel kernel 1240).
+// cover each other's pivots (N = 221: 840 us of an SM per slice and job, the
+// panel kernel alone on an SM 1160).
 SweepKernel sweep_kernel(Variant v, int N, bool few);  // negf_transmission.cu
 SweepKernel register_kernel(int N);          // negf_register.cu, up to RNMAX
 SweepKernel panel_kernel(int N);             // negf_panel.cu, up to PNMAX
