@@ -1012,6 +1012,7 @@ int negf_tri_solve(negf_ctx *ctx, const double *D, int32_t N, int32_t Nz, const 
     double2 *d_D = nullptr, *d_slab[2] = {}, *d_out[2] = {};
     int *d_nx = nullptr, *d_info = nullptr;
     RgfJob *d_job = nullptr;
+    cudaEvent_t ready = nullptr;  // the inputs are on the device
     int rc = 0, hinfo[2] = {0, 0};
     Geo g{};
     g.N = N; g.Nz = Nz; g.ld = round_up(N, 8);
@@ -1028,9 +1029,15 @@ int negf_tri_solve(negf_ctx *ctx, const double *D, int32_t N, int32_t Nz, const 
     CKT(cudaMalloc(&d_nx, sizeof(int) * N));
     CKT(cudaMalloc(&d_info, 2 * sizeof(int)));
     CKT(cudaMalloc(&d_job, sizeof(RgfJob)));
-    CKT(cudaMemset(d_nx, 0, sizeof(int) * N));
-    CKT(cudaMemset(d_job, 0, sizeof(RgfJob)));
-    CKT(cudaMemcpy(d_D, D, bytes, cudaMemcpyHostToDevice));
+    // The passes' streams do not wait for the default one, and a copy from
+    // pageable memory may return before its last part has arrived: the inputs
+    // go through the first stream, the second one waits for them.
+    CKT(cudaMemsetAsync(d_nx, 0, sizeof(int) * N, local[0].stream));
+    CKT(cudaMemsetAsync(d_job, 0, sizeof(RgfJob), local[0].stream));
+    CKT(cudaMemcpyAsync(d_D, D, bytes, cudaMemcpyHostToDevice, local[0].stream));
+    CKT(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    CKT(cudaEventRecord(ready, local[0].stream));
+    CKT(cudaStreamWaitEvent(local[1].stream, ready, 0));
     g.nx = g.ny = d_nx;
     {
         auto launch = [&](int p, double2 *slab) {
@@ -1085,6 +1092,7 @@ done:
         cudaFree(local[p].d_ws);
     }
     cudaFree(d_D); cudaFree(d_nx); cudaFree(d_info); cudaFree(d_job);
+    if (ready) cudaEventDestroy(ready);
     if (rc) return rc;
     return hinfo[0] ? hinfo[0] : hinfo[1];
 }
