@@ -20,7 +20,8 @@ namespace {
 constexpr int SP = 74;  // pitch of a shared block: k columns 8 banks apart for the A fragments
 constexpr int SC = 72;  // its columns
 
-// The block's inverse in natural order, to out (leading dimension ldo).
+// The block's inverse in natural order, to out (leading dimension ldo): scale a,
+// + scale where a pivot was (reg_eliminate).
 template <int PR, int CPW, int RPL, typename S>
 __device__ __forceinline__ void reg_store(const double2 (&a)[CPW][RPL], int N, const S &s, const int *rho, const int *kappa,
                                           const double2 *scale, double2 *out, int ldo) {
@@ -30,10 +31,14 @@ __device__ __forceinline__ void reg_store(const double2 (&a)[CPW][RPL], int N, c
         const int c = warp + RW * t;
         if (c < N) {
             double2 *col = out + (size_t)ldo * kappa[c];
+            const int one = s.unit[c];
 #pragma unroll
             for (int r = 0; r < PR; ++r) {
                 const int i = lane + 32 * r;
-                if (i < N) col[rho[i]] = zmul(scale[i], a[t][r]);
+                if (i < N) {
+                    const double2 sc = scale[i];
+                    col[rho[i]] = i == one ? zfma(sc, a[t][r], sc) : zmul(sc, a[t][r]);
+                }
             }
         }
     }

@@ -50,7 +50,8 @@ struct PanelSmem {
     double *gL, *gR, *kin; // [N]
     double *red;           // [PW]
     int *rho, *kappa, *cst;       // [N] maps of the slice
-    int *prow, *lin, *rows, *rest, *used;  // [N]
+    int *prow, *lin, *rows, *used;  // [N]
+    int *rest;             // [N] columns that a panel updates; between two inverses the pivot row of each storage column
     int *nrows, *info;
     int *piv;              // [3] pivot row of a step, by the step modulo 3
     int ldv;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void panel_factor(double2 (&a)[2][NRL], int N, int k0
 
 // Loads, eliminates and publishes the panel at k0: V into shared memory (a
 // team of one) or Vg[par] with its pivots (a larger team), the panel's own
-// columns V + e_p into the block.
+// columns V into the block (V + e_p less the 1: reg_eliminate).
 template <int NRL>
 __device__ __noinline__ void panel_rows_run(const PanelTeam &t, const PanelSmem &s, int N, int R, int k0, double2 *scale,
                                             int par) {
@@ -258,13 +259,12 @@ __device__ __noinline__ void panel_rows_run(const PanelTeam &t, const PanelSmem 
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int k = 16 * c + warp;
-        const int p = k < nb ? s.prow[k0 + k] : -1;
         double2 *col = t.A + (size_t)t.ld * (k < nb ? s.cst[k0 + k] : 0);
 #pragma unroll
         for (int r = 0; r < NRL; ++r) {
             const int i = lane + 32 * r;
             if (i < s.ldv - 2) V[(size_t)k * s.ldv + i] = a[c][r];
-            if (k < nb && i < R) col[i] = make_double2(i == p ? a[c][r].x + 1.0 : a[c][r].x, a[c][r].y);
+            if (k < nb && i < R) col[i] = a[c][r];
         }
     }
     if (t.size > 1) {
@@ -455,6 +455,7 @@ __device__ inline void panel_invert(const PanelTeam &t, const PanelSmem &s, int 
         s.rho[p] = tid;
         s.kappa[c] = b;
         s.cst[b] = c;
+        s.rest[c] = p;
     }
     __syncthreads();
 }
@@ -485,7 +486,7 @@ __device__ inline void panel_form(const PanelTeam &t, const PanelSmem &s, const 
     const double2 *vs = g.vhat + (size_t)g.W * g.H * b + g.ngx + g.W * g.ngy;
     for (int c = warp * t.size + t.rank; c < N; c += PW * t.size) {
         double2 *col = t.A + (size_t)t.ld * c;
-        const int kc = s.kappa[c];
+        const int kc = s.kappa[c], one = first ? -1 : s.rest[c];
         const double2 *vc = vs - s.lin[kc];
         for (int i0 = 0; i0 < N; i0 += 32 * 8) {
             double2 d[8], x[8];
@@ -507,7 +508,12 @@ __device__ inline void panel_form(const PanelTeam &t, const PanelSmem &s, const 
                         if (b == 0) y = zadd(y, s.sigL[m]);
                         if (b == g.Nz - 1) y = zadd(y, s.sigR[m]);
                     }
-                    col[i] = first ? y : zfms(scale[i], x[u], y);
+                    if (!first) {
+                        const double2 sc = scale[i];
+                        if (i == one) y = zsub(y, sc);
+                        y = zfms(sc, x[u], y);
+                    }
+                    col[i] = y;
                 }
             }
         }
