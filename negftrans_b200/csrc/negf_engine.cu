@@ -442,13 +442,18 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
     return 0;
 }
 
+// Workspace of njobs jobs of a slab kernel.
+size_t slab_ws_bytes(const SlabKernel &k, int N, int ld, int njobs) {
+    return sizeof(double2) * k.blocks * (size_t)ld * N * njobs;
+}
+
 int slab_launch(negf_ctx *c, const Geo &g, const RgfJob *d_jobs, int njobs, const double2 *d_D,
                 double2 *d_slabs, size_t sstride, int want, double2 *d_first, double2 *d_last,
                 int *d_info, cudaStream_t st) {
     const SlabKernel k = slab_kernel(g.N);
     if (!k.fn) return NEGF_ERR_UNSUPPORTED;
     size_t wstride = k.blocks * (size_t)g.ld * g.N;
-    int rc = ensure_ws(c, sizeof(double2) * wstride * njobs);
+    int rc = ensure_ws(c, slab_ws_bytes(k, g.N, g.ld, njobs));
     if (rc) return rc;
     double2 *ws = (double2 *)c->d_ws;
     int occ = 1;
@@ -1040,45 +1045,52 @@ int negf_tri_solve(negf_ctx *ctx, const double *D, int32_t N, int32_t Nz, const 
     CKT(cudaStreamWaitEvent(local[1].stream, ready, 0));
     g.nx = g.ny = d_nx;
     {
-        auto launch = [&](int p, double2 *slab) {
-            return slab_launch(&local[p], g, d_job, 1, d_D, slab, sstride, wants[p], p == 0 ? d_out[0] : nullptr,
-                               p == 1 ? d_out[1] : nullptr, d_info + p, local[p].stream);
+        // A pass has a slab, a workspace and a stream of its own; the second one
+        // takes the first one's, after it, where the device has no room for both.
+        int own[2] = {0, 1};
+        auto room = [&](int p) {
+            if (cudaMalloc(&d_slab[p], sizeof(double2) * sstride) != cudaSuccess) {
+                cudaGetLastError();
+                return (int)NEGF_ERR_CUDA;
+            }
+            return ensure_ws(&local[p], slab_ws_bytes(slab_kernel(N), N, g.ld, 1));
         };
-        // waits for pass p and copies its planes out of slab and d_out[p]
-        auto collect = [&](int p, const double2 *slab) {
-            if (cudaStreamSynchronize(local[p].stream) != cudaSuccess ||
+        auto launch = [&](int p) {
+            return slab_launch(&local[own[p]], g, d_job, 1, d_D, d_slab[own[p]], sstride, wants[p], p == 0 ? d_out[0] : nullptr,
+                               p == 1 ? d_out[1] : nullptr, d_info + p, local[own[p]].stream);
+        };
+        // waits for pass p and copies its planes out of its slab and d_out[p]
+        auto collect = [&](int p) {
+            if (cudaStreamSynchronize(local[own[p]].stream) != cudaSuccess ||
                 cudaMemcpy(&hinfo[p], d_info + p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
                 return NEGF_ERR_CUDA;
-            if ((wants[p] & WANT_D) && cudaMemcpy2D(diag, sizeof(double2) * N, slab, sizeof(double2) * g.ld, sizeof(double2) * N,
-                                                   (size_t)N * Nz, cudaMemcpyDeviceToHost) != cudaSuccess)
+            if ((wants[p] & WANT_D) &&
+                cudaMemcpy2D(diag, sizeof(double2) * N, d_slab[own[p]], sizeof(double2) * g.ld, sizeof(double2) * N,
+                             (size_t)N * Nz, cudaMemcpyDeviceToHost) != cudaSuccess)
                 return NEGF_ERR_CUDA;
             if (d_out[p] && cudaMemcpy(outs[p], d_out[p], bytes, cudaMemcpyDeviceToHost) != cudaSuccess) return NEGF_ERR_CUDA;
             return 0;
         };
-        bool pending[2] = {false, false};
         for (int p = 0; p < 2; ++p)
             if (wants[p] & (WANT_F | WANT_L)) CKT(cudaMalloc(&d_out[p], bytes));
         for (int p = 0; p < 2 && !rc; ++p) {
             if (!wants[p]) continue;
-            if (cudaMalloc(&d_slab[p], sizeof(double2) * sstride) != cudaSuccess) {
-                cudaGetLastError();
-                if (!pending[0]) { rc = NEGF_ERR_CUDA; break; }
-                break;  // no room for a second slab: the passes one after the other, below
+            rc = room(p);
+            if (rc && p == 1 && wants[0]) {
+                rc = 0;
+                own[1] = 0;
+                break;
             }
-            rc = launch(p, d_slab[p]);
-            pending[p] = !rc;
+            if (!rc) rc = launch(p);
         }
         // the reference zero-fills every plane (math_kernel.f90:75-77); this also
         // maps its pages while the GPU works
         if (diag) memset(diag, 0, bytes);
         if (first) memset(first, 0, bytes);
         if (last) memset(last, 0, bytes);
-        if (!rc && pending[0]) rc = collect(0, d_slab[0]);
-        if (!rc && wants[1] && !pending[1]) {
-            rc = launch(1, d_slab[0]);
-            pending[1] = !rc;
-        }
-        if (!rc && pending[1]) rc = collect(1, nullptr);
+        if (!rc && wants[0]) rc = collect(0);
+        if (!rc && wants[1] && own[1] == 0) rc = launch(1);
+        if (!rc && wants[1]) rc = collect(1);
     }
 #undef CKT
 done:

@@ -75,3 +75,24 @@ def test_register_inverse_keeps_its_last_bits(N, most):
         ref = diagonal_blocks_80_bits(D)
         err.append(float(np.sqrt(np.sum(abs(got["D"] - ref) ** 2) / np.sum(abs(ref) ** 2))) * 2.0 ** 53)
     assert np.mean(err) <= most
+
+
+# N = 800, two blocks: 61 MB of blocks, plane and slab, 61 MB of workspace, and as a choice 20 and 61 MB more for the
+# second pass beside the first
+@pytest.mark.parametrize("free_mb", [260, 175, 135])
+def test_tri_solve_in_little_memory(free_mb):
+    import torch
+    D = random_blocks(800, 2, 7)
+    ref, info = GreensFunction_tri_solver(D, "DL")
+    assert info == 0
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - free_mb * 1000000, dtype=torch.uint8, device="cuda")
+    try:
+        got, info = GreensFunction_tri_solver(D, "DL")
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert info == 0
+    for key in "DL":
+        assert (got[key] == ref[key]).all()
