@@ -27,6 +27,7 @@ struct negf_ctx {
     size_t ws_bytes = 0;
     double *d_E = nullptr, *d_tau = nullptr, *d_tau_jobs = nullptr;
     int *d_info = nullptr;
+    int *d_open = nullptr;    // most channels open at one energy of a transmission call
     int cap_E = 0, cap_jobs = 0;
     // mixed-precision path
     negf_mixed_policy mixed_policy{0.0, 0.0, 1e-7, 8, 0};
@@ -38,10 +39,10 @@ struct negf_ctx {
     double2 *d_voff = nullptr;
 };
 
-// FP64 sweeps of the listed jobs (energy index ie[q] into d_E, k-point ik[q])
-// of context c through the batch kernel: h_tau[q] the unweighted tau of job q,
-// h_info[q] its info; *ms the device time.  Synchronous on c->stream.
-int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const int *ik, int njobs,
+// FP64 sweeps of the listed jobs (energy index ie[q] into h_E and d_E, k-point
+// ik[q]) of context c through the batch kernel: h_tau[q] the unweighted tau of
+// job q, h_info[q] its info; *ms the device time.  Synchronous on c->stream.
+int negf_internal_fp64_jobs(negf_ctx *c, const double *h_E, const double *d_E, const int *ie, const int *ik, int njobs,
                             double *h_tau, int *h_info, float *ms);
 
 // The NEGF_MIXED transmission of all nE * nk jobs (job = ik * nE + ie, the

@@ -10,6 +10,7 @@
 //   k_accumulate    weighted sum of the diagonal blocks over the jobs of a
 //                   chunk (the accumulation loops of negf.f90:86-111,226-234)
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cmath>
@@ -41,6 +42,33 @@ __global__ void k_tau_reduce(const double *__restrict__ tau_jobs, const double *
     double t = 0.0;
     for (int ik = 0; ik < nk; ++ik) t += tau_jobs[(size_t)ik * nE + ie] * kw[ik];
     tau[ie] = t;
+}
+
+// *most = the channels of the left lead that are open at the highest of the
+// energies, over the k-points: an upper bound for every job of the call (a few
+// more under the lattice lead, whose channels close again at the band top).
+// A NaN energy has no open channel.  One CTA.
+__global__ void k_most_open(Geo g, const double *__restrict__ energies, int nE, int *most) {
+    __shared__ double top[32];
+    __shared__ int count;
+    double e = -CUDART_INF;
+    for (int i = threadIdx.x; i < nE; i += blockDim.x)
+        if (energies[i] > e) e = energies[i];
+    for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = e;
+    if (threadIdx.x == 0) *most = 0;
+    __syncthreads();
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) e = fmax(e, top[w]);
+    for (int ik = 0; ik < g.nk; ++ik) {
+        if (threadIdx.x == 0) count = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < g.N; i += blockDim.x) {
+            const double ax = g.ax[ik * g.N + i], ay = g.ay[ik * g.N + i];
+            if (ax * ax + ay * ay <= 2.0 * (e - g.V_L)) atomicAdd(&count, 1);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) *most = max(*most, count);
+    }
 }
 
 // out[o](i,j,k) (+)= sum_{q<gsz} coef[o*gsz+q] * ((slab_{o*gsz+q}(i,j,k) * 2) * dz^2)
@@ -325,6 +353,23 @@ int ensure_jobs(negf_ctx *c, int nE, int njobs) {
     return 0;
 }
 
+// The bound of k_most_open for energies on the host.
+int most_open(const negf_ctx *c, const double *E, int nE) {
+    double e = -INFINITY;
+    for (int i = 0; i < nE; ++i) e = E[i] > e ? E[i] : e;
+    int most = 0;
+    for (int ik = 0; ik < c->nk; ++ik) {
+        int n = 0;
+        for (int i = 0; i < c->N; ++i) {
+            const double ax = (double)(2 * c->nx[i]) * PI / c->Lx + c->kpt[3 * ik];
+            const double ay = (double)(2 * c->ny[i]) * PI / c->Ly + c->kpt[3 * ik + 1];
+            n += ax * ax + ay * ay <= 2.0 * (e - c->V_L);
+        }
+        most = std::max(most, n);
+    }
+    return most;
+}
+
 // Kernel variants by basis size: (panel width NB, rows per thread RPT,
 // CTAs per SM).  Up to 256 plane waves two CTAs share an SM.
 Variant pick_variant(int N) {
@@ -400,8 +445,8 @@ int shape_sweep(const void *fn, const SweepKernel &k, int sms, int njobs, size_t
 
 // The one-problem form of k on njobs jobs.
 int launch_one(const SweepKernel &k, Shape sh, Geo g, const double *d_E, int nE, int njobs, double2 *ws, size_t wstride,
-               double *d_tau_jobs, int *d_info, cudaStream_t st) {
-    void *args[] = {&g, &d_E, &nE, &njobs, &ws, &wstride, &d_tau_jobs, &d_info};
+               double *d_tau_jobs, int *d_info, Gate gate, cudaStream_t st) {
+    void *args[] = {&g, &d_E, &nE, &njobs, &ws, &wstride, &d_tau_jobs, &d_info, &gate};
     cudaLaunchAttribute at{};
     const cudaLaunchConfig_t lc = sweep_config(k, sh, &at, st);
     CK(cudaLaunchKernelExC(&lc, k.one, args));
@@ -418,6 +463,43 @@ int launch_batch(const SweepKernel &k, Shape sh, const Geo *d_geo, const BatchJo
     return 0;
 }
 
+// The kernels that a one-problem call may need, readied for njobs jobs.  The
+// choice hangs on the open channels, which the host does not know (the energies
+// are on the device): where it matters both kernels are launched, and the one
+// whose turn it is not ends at once (two launches, about 5 us of the 800 and more
+// that a sweep of these sizes takes).
+struct OneCall {
+    SweepKernel k[2];
+    Shape sh[2];
+    int n = 1, limit = 0;  // n == 2: k[0] up to `limit` open channels, k[1] above
+};
+int plan_one(Variant v, int N, int sms, int64_t njobs, size_t max_teams, OneCall *p) {
+    const int share = (int)(sms / std::max<int64_t>(njobs, 1));
+    p->k[0] = sweep_kernel(v, N, share, 0);
+    p->k[1] = sweep_kernel(v, N, share, N);
+    if (p->k[0].one != p->k[1].one) {
+        p->n = 2;
+        for (p->limit = 1; sweep_kernel(v, N, share, p->limit).one == p->k[0].one;) ++p->limit;
+    }
+    for (int i = 0; i < p->n; ++i)
+        if (int rc = shape_sweep(p->k[i].one, p->k[i], sms, (int)njobs, max_teams, &p->sh[i])) return rc;
+    return 0;
+}
+// ws: one workspace of wstride double2 (at least k.ws) for each CTA or team; d_open: one int.
+int run_one(const OneCall &p, const Geo &g, const double *d_E, int nE, int njobs, double2 *ws, size_t wstride,
+            double *d_tau_jobs, int *d_info, int *d_open, cudaStream_t st) {
+    if (p.n == 2) {
+        k_most_open<<<1, 256, 0, st>>>(g, d_E, nE, d_open);
+        CK(cudaGetLastError());
+    }
+    for (int i = 0; i < p.n; ++i) {
+        const Gate gate = p.n == 1 ? Gate{} : i == 0 ? Gate{d_open, 0, p.limit} : Gate{d_open, p.limit, INT32_MAX};
+        const size_t stride = wstride ? wstride : p.k[i].ws;
+        if (int rc = launch_one(p.k[i], p.sh[i], g, d_E, nE, njobs, ws, stride, d_tau_jobs, d_info, gate, st)) return rc;
+    }
+    return 0;
+}
+
 // CTAs of the slab kernel resident per SM for this N.
 int resident_ctas(int N) {
     const SlabKernel k = slab_kernel(N);
@@ -431,12 +513,13 @@ int transmission_launch(negf_ctx *c, const double *d_E, int nE, double *d_tau, d
     const int njobs = nE * c->nk;
     const Variant v = ctx_variant(c);
     if (v == VNONE) return NEGF_ERR_UNSUPPORTED;
-    const SweepKernel k = sweep_kernel(v, c->N, 2 * (int64_t)njobs <= c->num_sms);
-    Shape sh;
-    int rc = shape_sweep(k.one, k, c->num_sms, njobs, SIZE_MAX, &sh);
+    OneCall p;
+    int rc = plan_one(v, c->N, c->num_sms, njobs, SIZE_MAX, &p);
     if (rc) return rc;
-    if ((rc = ensure_ws(c, sizeof(double2) * k.ws * (sh.grid / sh.team)))) return rc;
-    if ((rc = launch_one(k, sh, make_geo(c), d_E, nE, njobs, (double2 *)c->d_ws, k.ws, d_tau_jobs, d_info, st))) return rc;
+    size_t ws = 0;
+    for (int i = 0; i < p.n; ++i) ws = std::max(ws, p.k[i].ws * (p.sh[i].grid / p.sh[i].team));
+    if ((rc = ensure_ws(c, sizeof(double2) * ws))) return rc;
+    if ((rc = run_one(p, make_geo(c), d_E, nE, njobs, (double2 *)c->d_ws, 0, d_tau_jobs, d_info, c->d_open, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(d_tau_jobs, c->d_kw, nE, c->nk, d_tau);
     CK(cudaGetLastError());
     return 0;
@@ -662,6 +745,7 @@ int negf_ctx_create(const negf_problem *p, int32_t device, negf_ctx **out) {
     CKC(cudaMalloc(&c->d_ax, sizeof(double) * ax.size()));
     CKC(cudaMalloc(&c->d_ay, sizeof(double) * ay.size()));
     CKC(cudaMalloc(&c->d_kw, sizeof(double) * kw.size()));
+    CKC(cudaMalloc(&c->d_open, sizeof(int)));
     CKC(cudaMemcpy(c->d_vhat, p->vhat, sizeof(double2) * nv, cudaMemcpyHostToDevice));
     CKC(cudaMemcpy(c->d_nx, p->nx, sizeof(int) * p->N, cudaMemcpyHostToDevice));
     CKC(cudaMemcpy(c->d_ny, p->ny, sizeof(int) * p->N, cudaMemcpyHostToDevice));
@@ -682,6 +766,7 @@ int negf_ctx_destroy(negf_ctx *c) {
     cudaFree(c->d_ws); cudaFree(c->d_E); cudaFree(c->d_tau); cudaFree(c->d_tau_jobs); cudaFree(c->d_info);
     cudaFree(c->d_mixed);
     cudaFree(c->d_voff);
+    cudaFree(c->d_open);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1113,7 +1198,7 @@ done:
 
 // FP64 re-runs for the mixed path: the listed (energy, k-point) jobs of one
 // context through the batch kernel.
-int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const int *ik, int njobs,
+int negf_internal_fp64_jobs(negf_ctx *c, const double *h_E, const double *d_E, const int *ie, const int *ik, int njobs,
                             double *h_tau, int *h_info, float *ms) {
     *ms = 0.f;
     if (njobs <= 0) return 0;
@@ -1121,8 +1206,12 @@ int negf_internal_fp64_jobs(negf_ctx *c, const double *d_E, const int *ie, const
     const Variant var = ctx_variant(c);
     if (var == VNONE) return NEGF_ERR_UNSUPPORTED;
     std::vector<BatchJob> jobs(njobs);
-    for (int q = 0; q < njobs; ++q) jobs[q] = BatchJob{0, ie[q], ik[q], 0};
-    const SweepKernel k = sweep_kernel(var, c->N, 2 * (int64_t)njobs <= c->num_sms);
+    std::vector<double> E(njobs);
+    for (int q = 0; q < njobs; ++q) {
+        jobs[q] = BatchJob{0, ie[q], ik[q], 0};
+        E[q] = h_E[ie[q]];
+    }
+    const SweepKernel k = sweep_kernel(var, c->N, c->num_sms / njobs, most_open(c, E.data(), njobs));
     Shape sh;
     int rc = shape_sweep(k.batch, k, c->num_sms, njobs, SIZE_MAX, &sh);
     if (rc) return rc;
@@ -1204,9 +1293,13 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         wide = wide || c->N > NT;
         middle += (int64_t)nE * c->nk;
     }
-    const bool few = wide || 2 * middle <= c0->num_sms;
+    const int share = std::max<int>(wide ? 2 : 0, (int)(c0->num_sms / std::max<int64_t>(middle, 1)));
     std::vector<const void *> kernels(nctx);
-    for (int p = 0; p < nctx; ++p) kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, few).batch;
+    std::vector<int> open(nctx);
+    for (int p = 0; p < nctx; ++p) {
+        open[p] = most_open(ctxs[p], energies, nE);
+        kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, share, open[p]).batch;
+    }
     for (int first = 0; first < nctx && !rc; ++first) {
         std::vector<int> members;
         for (int p = 0; p < nctx; ++p)
@@ -1215,11 +1308,9 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         std::vector<Geo> geos;
         std::vector<BatchJob> jobs;
         std::vector<double> cost;
-        int nmax = 0;
         for (int m = 0; m < (int)members.size(); ++m) {
             negf_ctx *c = ctxs[members[m]];
             geos.push_back(make_geo(c));
-            nmax = std::max(nmax, c->N);
             for (int ik = 0; ik < c->nk; ++ik)
                 for (int ie = 0; ie < nE; ++ie) {
                     jobs.push_back(BatchJob{m, ie, ik, 0});
@@ -1233,7 +1324,13 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         std::vector<BatchJob> sorted(jobs.size());
         for (size_t q = 0; q < order.size(); ++q) sorted[q] = jobs[order[q]];
         const int njobs = (int)sorted.size();
-        const SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), nmax, few);
+        // the members' kernel with the memory that the largest basis needs
+        SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), ctxs[first]->N, share, open[first]);
+        for (int p : members) {
+            const SweepKernel m = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, share, open[p]);
+            k.smem = std::max(k.smem, m.smem);
+            k.ws = std::max(k.ws, m.ws);
+        }
         Shape sh;
         if ((rc = shape_sweep(k.batch, k, c0->num_sms, njobs, SIZE_MAX, &sh))) break;
         if ((rc = ensure_ws(c0, sizeof(double2) * k.ws * (sh.grid / sh.team)))) break;
@@ -1657,9 +1754,8 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
 
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const SweepKernel k = sweep_kernel(v, N, 2 * njobs <= (size_t)sms);
-    Shape sh;
-    if ((rc = shape_sweep(k.one, k, sms, (int)njobs, cap, &sh))) return rc;
+    OneCall p;
+    if ((rc = plan_one(v, N, sms, (int64_t)njobs, cap, &p))) return rc;
 
     const int nkv = std::max(N * nk, nk);
     k_noalloc_kvectors<<<(nkv + 255) / 256, 256, 0, st>>>(d_nx, d_ny, d_kpt, N, nk, Lx, Ly, ax, ay, kw);
@@ -1674,7 +1770,7 @@ extern "C" int negf_transmission_noalloc(int32_t N, int32_t Nz, int32_t ngx, int
     g.c2 = 2 * (g.delta * g.delta);
     g.V_L = V_L; g.V_R = V_R; g.eta = eta;
     g.lead_model = 0;
-    if ((rc = launch_one(k, sh, g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info, st))) return rc;
+    if ((rc = run_one(p, g, d_energies, nE, (int)njobs, ws, wstride, tau_jobs, d_info, flag + 1, st))) return rc;
     k_tau_reduce<<<(nE + 127) / 128, 128, 0, st>>>(tau_jobs, kw, nE, nk, d_tau);
     CK(cudaGetLastError());
     return NEGF_OK;

@@ -2421,7 +2421,7 @@ int negf_internal_mixed(negf_ctx *c, const double *h_E, const double *d_E, int n
     if (!f_ie.empty()) {
         std::vector<double> t64(f_ie.size());
         std::vector<int> i64(f_ie.size());
-        rc = negf_internal_fp64_jobs(c, d_E, f_ie.data(), f_ik.data(), (int)f_ie.size(), t64.data(), i64.data(),
+        rc = negf_internal_fp64_jobs(c, h_E, d_E, f_ie.data(), f_ik.data(), (int)f_ie.size(), t64.data(), i64.data(),
                                      &ms64);
         if (rc) return rc;
         for (size_t q = 0; q < f_ie.size(); ++q) {

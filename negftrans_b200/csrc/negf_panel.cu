@@ -18,8 +18,9 @@ __device__ inline PanelTeam make_team(double2 *ws, size_t wstride, int N) {
 
 __global__ void __launch_bounds__(PT, 1)
     k_panel(Geo g, const double *__restrict__ energies, int nE, int njobs, double2 *ws, size_t wstride,
-            double *tau_jobs, int *info_jobs) {
+            double *tau_jobs, int *info_jobs, Gate gate) {
     extern __shared__ __align__(256) unsigned char smem[];
+    if (gate.shut()) return;
     const PanelTeam t = make_team(ws, wstride, g.N);
     const PanelSmem s = carve_panel(smem, g.N, 0);
     for (int job = blockIdx.x / t.size; job < njobs; job += gridDim.x / t.size) {

@@ -10,7 +10,7 @@ namespace {
 template <int CPW, int RPL, int PR, int MINB>
 __global__ void __launch_bounds__(RT, MINB)
     k_register(Geo g, const double *__restrict__ energies, int nE, int njobs, double2 *, size_t,
-               double *tau_jobs, int *info_jobs) {
+               double *tau_jobs, int *info_jobs, Gate) {
     __shared__ RegSmem<32 * RPL, CPW> s;
     for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
         const int ie = job % nE, ik = job / nE;  // energy fastest: negf.f90:131-133

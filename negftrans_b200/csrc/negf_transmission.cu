@@ -60,8 +60,9 @@ __device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, d
 template <int NB, int RPT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_transmission(Geo g, const double *__restrict__ energies, int nE, int njobs, double2 *ws,
-                   size_t wstride, double *tau_jobs, int *info_jobs) {
+                   size_t wstride, double *tau_jobs, int *info_jobs, Gate gate) {
     extern __shared__ __align__(256) unsigned char smem[];
+    if (gate.shut()) return;
     Smem s = carve<NB>(smem, g.N);
     for (int i = threadIdx.x; i < g.N; i += NT) { s.nx[i] = g.nx[i]; s.ny[i] = g.ny[i]; }
     __syncthreads();
@@ -119,14 +120,15 @@ SweepKernel make(int N) {
 
 }  // namespace
 
-SweepKernel sweep_kernel(Variant v, int N, bool few) {
+SweepKernel sweep_kernel(Variant v, int N, int share, int open) {
     switch (v) {
         case V16x1: return make<16, 1, 2>(N);
         case V16x2: return make<16, 2, 1>(N);
         case V8x4: return make<8, 4, 1>(N);
         case VCHIP:
             if (N <= RNMAX) return register_kernel(N);
-            return few || N > NT ? panel_kernel(N) : make<8, 1, 2>(N);
+            if ((share >= 2 || N > NT) && open <= panel_channels(N) * (share >= 8 ? 2 : 1)) return panel_kernel(N);
+            return N > NT ? make<16, 2, 1>(N) : make<8, 1, 2>(N);
         default: return SweepKernel{};
     }
 }

@@ -57,8 +57,6 @@ struct PanelSmem {
     int ldv;
 };
 
-__host__ __device__ inline int panel_rows(int N) { return 2 * N < PROWS ? round_up(2 * N, 8) : PROWS; }
-
 __host__ __device__ inline size_t panel_smem(int N) {
     const size_t n = round_up(N, 4);
     static_assert(3 * PROWS + 4 * PW <= PB * PCP, "the exchange buffers fit in B");

@@ -10,9 +10,16 @@ struct BatchJob {
     int prob, ie, ik, pad;
 };
 
+// A kernel that has nothing to do unless lo <= *open < hi (open null: always runs).
+struct Gate {
+    const int *open = nullptr;
+    int lo = 0, hi = 0;
+    __device__ bool shut() const { return open && (*open < lo || *open >= hi); }
+};
+
 // A transmission kernel in its two forms, of one signature for every variant:
 //   one    (Geo, const double *energies, int nE, int njobs, double2 *ws, size_t wstride,
-//           double *tau_jobs, int *info_jobs): the nE * nk jobs of one problem, energy fastest
+//           double *tau_jobs, int *info_jobs, Gate): the nE * nk jobs of one problem, energy fastest
 //   batch  (const Geo *, const BatchJob *, int njobs, const double *energies, double2 *ws,
 //           size_t wstride, double *tau_jobs, int *info_jobs, int *counter): jobs of several
 //           problems, taken in order from a counter
@@ -26,20 +33,32 @@ struct SweepKernel {
 
 // The variants of negf_set_variant.  0 .. 2 keep the block in global memory:
 // (panel width NB, rows per thread RPT, CTAs per SM), two CTAs per SM up to 256
-// plane waves.  3 is the family below, by basis size and number of jobs.
+// plane waves.  3 is the family below, by basis size, jobs and open channels.
 enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, VCHIP = 3, VNONE = 4 };
 
-// The kernel of a variant for a basis of N.  Variant 3: the block in registers
-// up to RNMAX; above, panels in registers and teams of CTAs if the jobs are
-// few (at most one per two SMs: nine jobs of N = 221, N_z = 160, 175 -> 86 ms in
-// teams of eight) or N > 256 (the next variant takes a whole SM as
-// well, at two rows per thread); otherwise 8 x 1 x 2, whose two jobs per SM
-// cover each other's pivots (N = 221: 840 us of an SM per slice and job, the
-// panel kernel alone on an SM 1160).
-SweepKernel sweep_kernel(Variant v, int N, bool few);  // negf_transmission.cu
+// The kernel of a variant for a basis of N, `share` SMs per job and at most
+// `open` channels open in the left lead.  Variant 3: the block in registers up
+// to RNMAX; above, panels in registers and teams of CTAs if the jobs are few
+// (two SMs each, or more: nine jobs of N = 221, N_z = 160, 175 -> 86 ms in teams
+// of eight) or N > 256 (148 jobs of N = 257, N_z = 6, 14.5 ms in 16 x 2 x 1, which
+// takes a whole SM as well, 10.7 in panels; N = 272 15.2 and 12.8); otherwise
+// 8 x 1 x 2, whose two jobs per SM cover each other's pivots (N = 221: 840 us of
+// an SM per slice and job, the panel kernel alone on an SM 1160).
+//
+// A block of the panel kernel has room for panel_channels(N) channels; more
+// take another sweep each time, where the other kernels only carry a wider
+// product.  One pass always gains; a second one only in the largest teams
+// (nine jobs of N = 257, 80 channels 12.3 -> 8.5 ms, 36 jobs 12.6 and 12.3, 148
+// jobs 15.7 and 23.2; N = 272 with all open 16.6 and 29.1, 20.4 and 78.1), so
+// that share >= 8 allows two passes, and every other call one.
+SweepKernel sweep_kernel(Variant v, int N, int share, int open);  // negf_transmission.cu
 SweepKernel register_kernel(int N);          // negf_register.cu, up to RNMAX
 SweepKernel panel_kernel(int N);             // negf_panel.cu, up to PNMAX
+// PNMAX: the block, its factor and one chunk of pivot rows in 227 KB of shared
+// memory, 320 rows of it in registers.
 constexpr int RNMAX = 72, PNMAX = 272;
+__host__ __device__ inline int panel_rows(int N) { return 2 * N < 320 ? round_up(2 * N, 8) : 320; }
+inline int panel_channels(int N) { return panel_rows(N) - N; }
 
 struct RgfJob {
     double e_re, e_im;  // complex energy of the solve, E + i*eta already added

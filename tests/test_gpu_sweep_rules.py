@@ -6,7 +6,9 @@ mode's bound (tests/test_gpu_parity.py).
 import numpy as np
 import pytest
 
-from negftrans_b200.negf import GreensFunction_tri_solver
+from negftrans_b200 import prepare as P
+from negftrans_b200 import workloads as W
+from negftrans_b200.negf import Engine, GreensFunction_tri_solver, transmission_batch
 
 pytestmark = pytest.mark.gpu
 RTOL, ATOL = 1e-9, 1e-12
@@ -96,3 +98,66 @@ def test_tri_solve_in_little_memory(free_mb):
     assert info == 0
     for key in "DL":
         assert (got[key] == ref[key]).all()
+
+
+def cut_problem(oracle, N, nz, nk=1, grid=64, seed=1000):
+    """The first N plane waves of a larger circular basis; the largest kinetic energy of theirs."""
+    V = W.MSTAR * W.qpc_potential(grid, grid, nz, 100.0, nz * 1.0, 0.050, 15.0, max(nz / 6.0, 1.0), disorder=0.002,
+                                  seed=seed)
+    pr = P.prepare(W._deck(nz * 10.0, (N + 12) * 4.9e-5, 30.0, 16, nk=nk), V)
+    assert pr.N >= N
+    args = (np.ascontiguousarray(pr.nx[:N]), np.ascontiguousarray(pr.ny[:N])) + pr.engine_args()[2:]
+    kin = 0.5 * ((2 * np.pi * pr.nx[:N] / pr.atomic.LX) ** 2 + (2 * np.pi * pr.ny[:N] / pr.atomic.LY) ** 2)
+    return args, oracle.Problem(*args), kin.max()
+
+
+# a block of the panel kernel has 320 - N rows for channels: at and past that, few jobs and many, every entry
+@pytest.mark.parametrize("N,nE,variant", [(240, 40, 0), (256, 74, 0), (257, 40, 1), (272, 150, 1)])
+def test_many_open_channels_take_one_sweep(oracle, N, nE, variant):
+    import torch
+    args, op, kmax = cut_problem(oracle, N, nz=3)
+    E = np.linspace(1.1, 1.2, nE) * kmax
+    E[1] = np.nan
+    check = [0, 2, nE - 1]
+    ref, _ = oracle.transmission_jobs(op, E[check], nthreads=8)
+    with Engine(*args) as eng:
+        best = {}
+        for v in (-1, variant):
+            eng.set_variant(v)
+            ms = []
+            for _ in range(4):
+                tau, info = eng.transmission(E)
+                ms.append(eng.last_stats.device_ms)
+                assert info > 0 and eng.last_stats.n_singular == 1 and eng.last_stats.first_bad_job == 1
+                np.testing.assert_allclose(tau[check], ref, rtol=RTOL, atol=ATOL)
+            best[v] = min(ms)
+            if v < 0:
+                dE = torch.tensor(E, device="cuda")
+                dt = torch.zeros(nE, dtype=torch.float64, device="cuda")
+                torch.cuda.synchronize()
+                eng.transmission_device(dE.data_ptr(), nE, dt.data_ptr())
+                torch.cuda.synchronize()
+                assert (dt.cpu().numpy()[check] == tau[check]).all()
+        eng.set_variant(-1)
+        both, info, _ = transmission_batch([eng], E)
+        np.testing.assert_allclose(both[0][check], ref, rtol=RTOL, atol=ATOL)
+    # several sweeps per job take two to four times as long
+    assert best[-1] <= 1.4 * best[variant]
+
+
+# about as many channels as a block has room for, on both sides of it; one and two passes in the largest teams
+@pytest.mark.parametrize("N,nE", [(200, 4), (221, 30), (260, 4), (272, 20)])
+def test_open_channels_at_the_edge_of_the_block(oracle, N, nE):
+    args, op, kmax = cut_problem(oracle, N, nz=2)
+    kin = np.sort(0.5 * ((2 * np.pi * args[0] / args[3]) ** 2 + (2 * np.pi * args[1] / args[4]) ** 2))
+    for passes in (1, 2):
+        room = min(N, passes * (320 - N))
+        for top in (0.5 * (kin[room - 2] + kin[room - 1]), kin[min(room, N - 1)] * (1 + 1e-9) + 1e-9):
+            E = np.linspace(0.3, 1.0, nE) * top
+            ref, _ = oracle.transmission_jobs(op, E, nthreads=8)
+            with Engine(*args) as eng:
+                tau, info = eng.transmission(E)
+                both, _, _ = transmission_batch([eng], E)
+            assert info == 0
+            np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
+            np.testing.assert_allclose(both[0], ref, rtol=RTOL, atol=ATOL)
