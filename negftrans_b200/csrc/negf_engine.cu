@@ -103,11 +103,14 @@ __global__ void k_accumulate(const double2 *__restrict__ slabs, size_t sstride, 
 // G is binned on the difference n_a - n_b in shared memory, then transformed
 // along x (UC rows of u at a time) and along y.  Writes Im(diag) * scale
 // (main.f90:341-351) to dens, or the complex diagonal to cdiag.
-// Bound by the transforms' FP64 work.  A bin is summed by one thread, over a in
-// order with b looked up from n_a - d (adding G into the bins needs a
-// compare-and-swap loop per FP64 add in shared memory), and the phases advance
-// by one addition instead of a remainder per term: 60 thousand slices of N = 69
-// on a 64 x 64 grid 7.7 -> 6.1 ms.
+// Bound by the bins up to a few hundred plane waves (about five lookups per pair
+// of them), then by the reads of G.  A bin is summed by one thread, over b in
+// order with a looked up from n_b + d: neighbouring threads read neighbouring
+// rows, eight loads in flight each, and no adds into shared memory, which FP64
+// does by compare-and-swap loops.  The phases advance by one addition instead
+// of a remainder per term.  Against compare-and-swap sums and remainders: 592
+// slices of N = 69 on a 64 x 64 grid 94 -> 69 us, of N = 221 317 -> 277 us; 296 of
+// N = 500 on 128 x 128 1.12 -> 0.93 ms, 148 of N = 797 2.11 -> 1.84 ms.
 constexpr int PT_THREADS = 256;
 constexpr int PT_UC = 16;
 
@@ -138,21 +141,35 @@ __global__ void __launch_bounds__(PT_THREADS)
         twy[m] = make_double2(cs, sn);
     }
     __syncthreads();
+    bool dup = false;  // a basis may hold a vector more than once
     for (int a = threadIdx.x; a < N; a += PT_THREADS) {
         sx[a] = nx[a] + mx;
         sy[a] = ny[a] + my;
         also[a] = atomicExch(at + sx[a] + LX * sy[a], a);
+        dup |= also[a] >= 0;
     }
-    __syncthreads();
+    const bool twice = __syncthreads_or(dup);
     for (int e = threadIdx.x; e < BX * BY; e += PT_THREADS) {
         const int dx = e % BX - 2 * mx, dy = e / BX - 2 * my;
         double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 4
-        for (int a = 0; a < N; ++a) {
-            const int bx = sx[a] - dx, by = sy[a] - dy;
-            int b = (unsigned)bx < (unsigned)LX && (unsigned)by < (unsigned)LY ? at[bx + LX * by] : -1;
-            for (; b >= 0; b = also[b]) acc = zadd(acc, Gk[a + (size_t)ldg * b]);
+        auto row = [&](int b) {  // a row a with n_a - n_b = (dx, dy)
+            const int ax = sx[b] + dx, ay = sy[b] + dy;
+            return (unsigned)ax < (unsigned)LX && (unsigned)ay < (unsigned)LY ? at[ax + LX * ay] : -1;
+        };
+        for (int b0 = 0; b0 < N; b0 += 8) {
+            double2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int a = b0 + u < N ? row(b0 + u) : -1;
+                v[u] = a >= 0 ? Gk[a + (size_t)ldg * (b0 + u)] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc = zadd(acc, v[u]);
         }
+        if (twice)
+            for (int b = 0; b < N; ++b)
+                for (int a = row(b); a >= 0; a = also[a])
+                    if (also[a] >= 0) acc = zadd(acc, Gk[also[a] + (size_t)ldg * b]);
         bin[e] = acc;
     }
     __syncthreads();

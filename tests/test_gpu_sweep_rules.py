@@ -161,3 +161,24 @@ def test_open_channels_at_the_edge_of_the_block(oracle, N, nE):
             assert info == 0
             np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
             np.testing.assert_allclose(both[0], ref, rtol=RTOL, atol=ATOL)
+
+
+# bins of few and of many plane waves, on both sides of a batch of eight; an elongated basis; vectors held twice or more
+@pytest.mark.parametrize("N,mx,my,twice", [(1, 0, 0, 0), (7, 1, 1, 0), (69, 5, 4, 0), (97, 40, 1, 0), (300, 9, 10, 0),
+                                           (40, 4, 3, 5), (9, 0, 0, 0)])
+def test_real_space_density(N, mx, my, twice):
+    from negftrans_b200.grid import Greensfunction_PlanewaveToReal
+    rng = np.random.default_rng(N)
+    pos = [(x, y) for y in range(-my, my + 1) for x in range(-mx, mx + 1)]
+    pick = np.sort(rng.choice(len(pos), min(N, len(pos)), replace=False))
+    pick = np.concatenate([pick, rng.choice(pick, N - len(pick)), ])
+    pick[:twice] = pick[-1]
+    nx, ny = np.array([pos[i] for i in pick], np.int32).T
+    Nx, Ny, nz = 2 * mx + 3, 2 * my + 2, 3
+    G = np.asfortranarray(rng.standard_normal((N, N, nz)) + 1j * rng.standard_normal((N, N, nz)))
+    ref = np.stack([Greensfunction_PlanewaveToReal(G[:, :, k], nx, ny, Nx, Ny) for k in range(nz)], 2)
+    with Engine(nx, ny, np.zeros((4 * mx + 1, 4 * my + 1, nz), complex), 1.0, 1.0, 1.0, 0.0, 0.0, 1e-6,
+                [[0, 0, 1]]) as eng:
+        got = eng.dm_real(G, Nx, Ny, 1.0, 1.0, float(nz))
+    # at most N^2 terms a point: sums of random signs, far inside N^2 eps
+    assert np.max(np.abs(got - ref.imag)) <= 1e-12 * N
