@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(PT_THREADS)
     double2 *twx = T + (size_t)PT_UC * BY;               // [Nx] e^{+2 pi i m/Nx}
     double2 *twy = twx + Nx;                             // [Ny]
     int *at = (int *)(twy + Ny);                         // [LY][LX] a basis index of (n, m), -1: none
-    int *sx = at + LX * LY, *sy = sx + N;                // [N] the basis
-    int *also = sy + N;                                  // [N] another index of the same (n, m), -1: none
+    short *sx = (short *)(at + LX * LY), *sy = sx + N;   // [N] the basis
+    short *also = sy + N;                                // [N] another index of the same (n, m), -1: none
     const int k = blockIdx.x;
     const double2 *Gk = G + gstride * k;
     for (int e = threadIdx.x; e < LX * LY; e += PT_THREADS) at[e] = -1;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(PT_THREADS)
     for (int a = threadIdx.x; a < N; a += PT_THREADS) {
         sx[a] = nx[a] + mx;
         sy[a] = ny[a] + my;
-        also[a] = atomicExch(at + sx[a] + LX * sy[a], a);
+        also[a] = (short)atomicExch(at + sx[a] + LX * sy[a], a);
         dup |= also[a] >= 0;
     }
     const bool twice = __syncthreads_or(dup);
@@ -213,14 +213,16 @@ __global__ void __launch_bounds__(PT_THREADS)
     }
 }
 
-// Shared memory of the bins and tables; the index lists come on top (at most
-// 27 KB where these fit 200 KB).
+// Shared memory of the bins and tables; the index lists come on top.  Where the
+// tables fit 200 KB, LX LY is at most 4261 (all of the basis along one axis, on
+// the smallest grid), so with 1024 plane waves the lists take up to 22.7 KB of
+// the 27 KB left.
 size_t ptor_smem(int mx, int my, int Nx, int Ny) {
     const size_t BX = 4 * (size_t)mx + 1, BY = 4 * (size_t)my + 1;
     return sizeof(double2) * (BX * BY + PT_UC * BY + Nx + Ny);
 }
 size_t ptor_lists(int N, int mx, int my) {
-    return sizeof(int) * ((2 * (size_t)mx + 1) * (2 * (size_t)my + 1) + 3 * (size_t)N);
+    return sizeof(int) * (2 * (size_t)mx + 1) * (2 * (size_t)my + 1) + 3 * sizeof(short) * (size_t)N;
 }
 
 // LDOS_grid_converter (tools.f90:18-40) applied to one energy's real-space

@@ -182,3 +182,18 @@ def test_real_space_density(N, mx, my, twice):
         got = eng.dm_real(G, Nx, Ny, 1.0, 1.0, float(nz))
     # at most N^2 terms a point: sums of random signs, far inside N^2 eps
     assert np.max(np.abs(got - ref.imag)) <= 1e-12 * N
+
+
+def test_real_space_density_of_the_longest_basis():
+    """1000 plane waves over 4241 along x: tables of 199 KB and the index lists on top."""
+    from negftrans_b200.grid import Greensfunction_PlanewaveToReal
+    rng = np.random.default_rng(3)
+    N, mx = 1000, 2120
+    nx = np.sort(rng.choice(2 * mx + 1, N, replace=False)).astype(np.int32) - mx
+    nx[0], nx[-1] = -mx, mx
+    ny = np.zeros(N, np.int32)
+    G = np.asfortranarray(rng.standard_normal((N, N, 2)) + 1j * rng.standard_normal((N, N, 2)))
+    ref = Greensfunction_PlanewaveToReal(G, nx, ny, 2 * mx + 3, 1)
+    with Engine(nx, ny, np.zeros((4 * mx + 1, 1, 2), complex), 1.0, 1.0, 1.0, 0.0, 0.0, 1e-6, [[0, 0, 1]]) as eng:
+        got = eng.dm_real(G, 2 * mx + 3, 1, 1.0, 1.0, 2.0)
+    assert np.max(np.abs(got - ref.imag)) <= 1e-12 * N
