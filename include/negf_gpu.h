@@ -186,7 +186,8 @@ int negf_get_mixed_stats(const negf_ctx *ctx, negf_mixed_stats *stats);
 /* negf_transmission for nctx problems at once -- e.g. one per k-point with a
  * per-k basis, or several devices of different length -- on the device of
  * ctxs[0] (all contexts must share it).  One persistent launch per kernel
- * variant takes the (problem, E, k) jobs largest-first from a counter.  The
+ * takes the (problem, E, k) jobs largest-first from a counter; the launches
+ * run side by side where the device has room for their workspaces.  The
  * energies are shared; tau[p*nE + e] = sum over the k-points of ctxs[p] of
  * weight * tau.  A multi-problem generalisation of the job loop of
  * main.f90:384-407 (the reference runs one problem per process). */

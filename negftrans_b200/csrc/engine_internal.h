@@ -12,6 +12,7 @@ struct negf_ctx {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    std::vector<cudaStream_t> side;  // of a batch's kernels beside the first one
     int N = 0, Nz = 0, ld = 0, ngx = 0, ngy = 0, nk = 0;
     double Lx = 0, Ly = 0, Lz = 0, V_L = 0, V_R = 0, eta = 0;
     int lead_model = 0;

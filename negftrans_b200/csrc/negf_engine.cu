@@ -16,7 +16,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "engine_internal.h"
@@ -440,9 +442,10 @@ cudaLaunchConfig_t sweep_config(const SweepKernel &k, Shape sh, cudaLaunchAttrib
 
 // Readies fn (one of k's two forms) and shapes its launch for njobs jobs, at
 // most max_teams of them at once.  The team is the largest that still runs
-// every job at once: a smaller one would leave SMs idle, a larger one would
-// make jobs wait, and a team's time falls by less than its size.
-int shape_sweep(const void *fn, const SweepKernel &k, int sms, int njobs, size_t max_teams, Shape *sh) {
+// every job of the call at once (njobs, or more with other kernels beside this
+// one): a smaller one would leave SMs idle, a larger one would make jobs wait,
+// and a team's time falls by less than its size.
+int shape_sweep(const void *fn, const SweepKernel &k, int sms, int njobs, size_t max_teams, Shape *sh, int64_t of_call = 0) {
     int occ = 1;
     int rc = prep_kernel(fn, k.threads, k.smem, &occ);
     if (rc) return rc;
@@ -453,7 +456,7 @@ int shape_sweep(const void *fn, const SweepKernel &k, int sms, int njobs, size_t
         const cudaLaunchConfig_t lc = sweep_config(k, *sh, &at, nullptr);
         int most = 0;
         CK(cudaOccupancyMaxActiveClusters(&most, fn, &lc));
-        if (njobs <= most) {
+        if (std::max<int64_t>(njobs, of_call) <= most) {
             teams = (size_t)most;
             break;
         }
@@ -786,6 +789,7 @@ int negf_ctx_destroy(negf_ctx *c) {
     cudaFree(c->d_mixed);
     cudaFree(c->d_voff);
     cudaFree(c->d_open);
+    for (cudaStream_t s : c->side) cudaStreamDestroy(s);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1281,6 +1285,61 @@ extern "C" int negf_get_mixed_stats(const negf_ctx *c, negf_mixed_stats *s) {
 }
 
 // ------------------------------------------------------ batches of problems
+namespace {
+// The sweeps of a batch that share a kernel.
+struct BatchGroup {
+    SweepKernel k;                // with the memory that the largest basis needs
+    Shape sh;
+    std::vector<int> members;     // problems
+    std::vector<BatchJob> jobs;   // problem-major, then k-point, energy fastest
+    std::vector<int> order;       // of the launch, largest sweeps first
+    double longest = 0;           // N^3 Nz of the largest sweep
+    size_t ws_at = 0, geo_at = 0, jobs_at = 0, tau_at = 0, info_at = 0, counter_at = 0;  // bytes into the buffers
+    size_t ws_bytes() const { return sizeof(double2) * k.ws * (sh.grid / sh.team); }
+};
+
+// When a launch of the given sweeps ends, one SM after the other: longest first,
+// each to the slot that is free first, `slots` of them on an SM, `unit` times
+// its cost each.  at: when each SM is free, before and after.
+void pack(std::vector<double> cost, int slots, double unit, std::vector<double> *at) {
+    typedef std::pair<double, int> Slot;  // free at, SM
+    std::priority_queue<Slot, std::vector<Slot>, std::greater<Slot>> next;
+    for (int s = 0; s < (int)at->size(); ++s)
+        for (int u = 0; u < slots; ++u) next.push(Slot((*at)[s], s));
+    std::sort(cost.begin(), cost.end(), std::greater<double>());
+    for (double c : cost) {
+        const Slot f = next.top();
+        next.pop();
+        (*at)[f.second] = std::max((*at)[f.second], f.first + unit * c);
+        next.push(Slot(f.first + unit * c, f.second));
+    }
+}
+
+// Whether the sweeps of 73 .. 256 plane waves go to the panel kernel with those
+// above 256, at any number of jobs.  Beside a panel launch of its own the other
+// kernel, 8 x 1 x 2, runs them with two on an SM: less of the chip for a sweep,
+// but longer from slice to slice.  So the panels win where the longest sweeps
+// set the time, and lose where there is work for the whole chip.  Which it is
+// comes from packing both ways, at 1000 us a slice of N = 221 in panels and
+// 1640 beside another sweep (N^3 at other sizes).  Measured, one kernel against
+// two: 16 bases of 180-263 with 15, 30 and 60 slices, 288, 576, 1152 and 2304
+// sweeps 97, 143, 280 and 558 ms against 145, 147, 255 and 505; 1800 sweeps of
+// N = 221 with 150 of N = 260 198 against 166.  Of 41 such batches, N from 80 to
+// 270, one took a way that was more than 1 % the slower (by 7 %).
+bool panels_for_all(const std::vector<double> &middle, const std::vector<double> &wide, int sms) {
+    if (middle.empty() || wide.empty()) return false;
+    const double unit = 1.0 / (221.0 * 221.0 * 221.0);
+    std::vector<double> one(sms, 0.0), two(sms, 0.0), all = middle;
+    all.insert(all.end(), wide.begin(), wide.end());
+    pack(all, 1, 1000 * unit, &one);
+    const bool wide_first = *std::max_element(wide.begin(), wide.end()) >= *std::max_element(middle.begin(), middle.end());
+    for (int turn = 0; turn < 2; ++turn)
+        if ((turn == 0) == wide_first) pack(wide, 1, 1000 * unit, &two);
+        else pack(middle, 2, 1640 * unit, &two);
+    return *std::max_element(one.begin(), one.end()) < *std::max_element(two.begin(), two.end());
+}
+}  // namespace
+
 extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, const double *energies, int32_t nE,
                                        double *tau, negf_stats *stats) {
     if (!ctxs || nctx < 1 || !energies || !tau || nE < 1) return NEGF_ERR_ARG;
@@ -1288,119 +1347,125 @@ extern "C" int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, cons
         if (!ctxs[p] || ctxs[p]->device != ctxs[0]->device) return NEGF_ERR_ARG;
     negf_ctx *c0 = ctxs[0];
     if (cudaSetDevice(c0->device) != cudaSuccess) return NEGF_ERR_CUDA;
-    cudaStream_t st = c0->stream;
     std::fill(tau, tau + (size_t)nctx * nE, 0.0);
-    double *d_E = nullptr;
-    if (cudaMalloc(&d_E, sizeof(double) * nE) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
-    if (cudaMemcpyAsync(d_E, energies, sizeof(double) * nE, cudaMemcpyHostToDevice, st) != cudaSuccess) {
-        cudaFree(d_E);
-        return NEGF_ERR_CUDA;
-    }
-    std::vector<int> info_all;
-    double ms_all = 0;
-    int rc = 0;
-    // One launch per kernel, its problems in the order given.  The middle sizes
-    // (RNMAX < N <= PNMAX, chosen by N) stay together: with bases on both sides
-    // of NT, or few jobs, all of them run in the panel kernel, since a second
-    // launch would wait for the first one's last sweep (48 problems of 180-263
-    // plane waves, 576 sweeps: 272 ms in two launches, 143 in one).
-    bool wide = false;
-    int64_t middle = 0;
+    // the kernel of each problem
+    std::vector<int> open(nctx);
+    std::vector<double> middle, wide;
+    int64_t large = 0;  // sweeps above RNMAX; the others are done long before those
     for (int p = 0; p < nctx; ++p) {
         const negf_ctx *c = ctxs[p];
-        if (ctx_variant(c) != VCHIP || c->N <= RNMAX) continue;
-        wide = wide || c->N > NT;
-        middle += (int64_t)nE * c->nk;
+        open[p] = most_open(c, energies, nE);
+        if (c->N > RNMAX) large += (int64_t)nE * c->nk;
+        if (ctx_variant(c) != VCHIP || c->N <= RNMAX || open[p] > panel_channels(c->N)) continue;
+        std::vector<double> &v = c->N > NT ? wide : middle;
+        v.insert(v.end(), (size_t)nE * c->nk, (double)c->N * c->N * c->N * c->Nz);
     }
-    const int share = std::max<int>(wide ? 2 : 0, (int)(c0->num_sms / std::max<int64_t>(middle, 1)));
-    std::vector<const void *> kernels(nctx);
-    std::vector<int> open(nctx);
+    int share = (int)(c0->num_sms / std::max<int64_t>(large, 1));
+    if (share < 2 && panels_for_all(middle, wide, c0->num_sms)) share = 2;
+    auto kernel = [&](int p) { return sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, share, open[p]); };
+    std::vector<BatchGroup> groups;
     for (int p = 0; p < nctx; ++p) {
-        open[p] = most_open(ctxs[p], energies, nE);
-        kernels[p] = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, share, open[p]).batch;
+        const negf_ctx *c = ctxs[p];
+        const SweepKernel k = kernel(p);
+        auto g = std::find_if(groups.begin(), groups.end(), [&](const BatchGroup &x) { return x.k.batch == k.batch; });
+        if (g == groups.end()) {
+            groups.emplace_back();
+            g = groups.end() - 1;
+            g->k = k;
+        }
+        g->k.smem = std::max(g->k.smem, k.smem);
+        g->k.ws = std::max(g->k.ws, k.ws);
+        g->longest = std::max(g->longest, (double)c->N * c->N * c->N * c->Nz);
+        for (int ik = 0; ik < c->nk; ++ik)
+            for (int ie = 0; ie < nE; ++ie) g->jobs.push_back(BatchJob{(int)g->members.size(), ie, ik, 0});
+        g->members.push_back(p);
     }
-    for (int first = 0; first < nctx && !rc; ++first) {
-        std::vector<int> members;
-        for (int p = 0; p < nctx; ++p)
-            if (kernels[p] == kernels[first]) members.push_back(p);
-        if (members[0] != first) continue;  // launched already
-        std::vector<Geo> geos;
-        std::vector<BatchJob> jobs;
-        std::vector<double> cost;
-        for (int m = 0; m < (int)members.size(); ++m) {
-            negf_ctx *c = ctxs[members[m]];
-            geos.push_back(make_geo(c));
-            for (int ik = 0; ik < c->nk; ++ik)
-                for (int ie = 0; ie < nE; ++ie) {
-                    jobs.push_back(BatchJob{m, ie, ik, 0});
-                    cost.push_back((double)c->N * c->N * c->N * c->Nz);
-                }
-        }
-        // largest sweeps first, so the last wave holds the short ones
-        std::vector<int> order(jobs.size());
-        for (size_t q = 0; q < order.size(); ++q) order[q] = (int)q;
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-        std::vector<BatchJob> sorted(jobs.size());
-        for (size_t q = 0; q < order.size(); ++q) sorted[q] = jobs[order[q]];
-        const int njobs = (int)sorted.size();
-        // the members' kernel with the memory that the largest basis needs
-        SweepKernel k = sweep_kernel(ctx_variant(ctxs[first]), ctxs[first]->N, share, open[first]);
-        for (int p : members) {
-            const SweepKernel m = sweep_kernel(ctx_variant(ctxs[p]), ctxs[p]->N, share, open[p]);
-            k.smem = std::max(k.smem, m.smem);
-            k.ws = std::max(k.ws, m.ws);
-        }
-        Shape sh;
-        if ((rc = shape_sweep(k.batch, k, c0->num_sms, njobs, SIZE_MAX, &sh))) break;
-        if ((rc = ensure_ws(c0, sizeof(double2) * k.ws * (sh.grid / sh.team)))) break;
-        Geo *d_geo = nullptr;
-        BatchJob *d_jobs = nullptr;
-        double *d_tj = nullptr;
-        int *d_info = nullptr, *d_counter = nullptr;
-        if (cudaMalloc(&d_geo, sizeof(Geo) * geos.size()) != cudaSuccess ||
-            cudaMalloc(&d_jobs, sizeof(BatchJob) * njobs) != cudaSuccess ||
-            cudaMalloc(&d_tj, sizeof(double) * njobs) != cudaSuccess ||
-            cudaMalloc(&d_info, sizeof(int) * njobs) != cudaSuccess ||
-            cudaMalloc(&d_counter, sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            rc = NEGF_ERR_NOMEM;
-        }
-        std::vector<double> tj(njobs);
-        std::vector<int> info(njobs);
-        float ms = 0.f;
-        if (!rc) {
-            if (cudaMemcpyAsync(d_geo, geos.data(), sizeof(Geo) * geos.size(), cudaMemcpyHostToDevice, st) ||
-                cudaMemcpyAsync(d_jobs, sorted.data(), sizeof(BatchJob) * njobs, cudaMemcpyHostToDevice, st) ||
-                cudaMemsetAsync(d_counter, 0, sizeof(int), st) || cudaEventRecord(c0->ev0, st))
-                rc = NEGF_ERR_CUDA;
-        }
-        if (!rc) {
-            rc = launch_batch(k, sh, d_geo, d_jobs, njobs, d_E, (double2 *)c0->d_ws, k.ws, d_tj, d_info, d_counter, st);
-            if (rc || cudaEventRecord(c0->ev1, st) ||
-                cudaMemcpyAsync(tj.data(), d_tj, sizeof(double) * njobs, cudaMemcpyDeviceToHost, st) ||
-                cudaMemcpyAsync(info.data(), d_info, sizeof(int) * njobs, cudaMemcpyDeviceToHost, st) ||
-                cudaStreamSynchronize(st) || cudaEventElapsedTime(&ms, c0->ev0, c0->ev1))
-                rc = NEGF_ERR_CUDA;
-        }
-        cudaFree(d_geo); cudaFree(d_jobs); cudaFree(d_tj); cudaFree(d_info); cudaFree(d_counter);
-        if (rc) break;
-        ms_all += ms;
-        // tau[p][e] = sum_k w_k tau(p, e, k), summed in k order (negf.f90:172)
-        std::vector<double> per(jobs.size());
-        for (size_t q = 0; q < order.size(); ++q) per[order[q]] = tj[q];
-        size_t q = 0;
-        for (int m = 0; m < (int)members.size(); ++m) {
-            negf_ctx *c = ctxs[members[m]];
-            const int pg = members[m];
-            for (int ik = 0; ik < c->nk; ++ik)
-                for (int ie = 0; ie < nE; ++ie, ++q) tau[(size_t)pg * nE + ie] += per[q] * c->kpt[3 * ik + 2];
-        }
-        for (size_t qq = 0; qq < order.size(); ++qq) info_all.push_back(info[qq]);
+    // The group with the longest sweep first, so that it starts on a free chip.
+    std::stable_sort(groups.begin(), groups.end(), [](const BatchGroup &x, const BatchGroup &y) { return x.longest > y.longest; });
+    int rc = 0;
+    size_t bytes = sizeof(double) * nE, ws = 0, most = 0;
+    auto take = [&](size_t n) {
+        const size_t at = (bytes + 255) / 256 * 256;
+        bytes = at + n;
+        return at;
+    };
+    for (BatchGroup &g : groups) {
+        if ((rc = shape_sweep(g.k.batch, g.k, c0->num_sms, (int)g.jobs.size(), SIZE_MAX, &g.sh, large))) return rc;
+        g.order.resize(g.jobs.size());
+        for (size_t q = 0; q < g.order.size(); ++q) g.order[q] = (int)q;
+        auto cost = [&](int q) {
+            const negf_ctx *c = ctxs[g.members[g.jobs[q].prob]];
+            return (double)c->N * c->N * c->N * c->Nz;
+        };
+        std::stable_sort(g.order.begin(), g.order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+        g.geo_at = take(sizeof(Geo) * g.members.size());
+        g.jobs_at = take(sizeof(BatchJob) * g.jobs.size());
+        g.counter_at = take(sizeof(int));
+        g.ws_at = ws;
+        ws += (g.ws_bytes() + 255) / 256 * 256;
+        most = std::max(most, g.ws_bytes());
     }
-    cudaFree(d_E);
+    const size_t in_bytes = bytes;
+    for (BatchGroup &g : groups) {
+        g.tau_at = take(sizeof(double) * g.jobs.size());
+        g.info_at = take(sizeof(int) * g.jobs.size());
+    }
+    // The groups run side by side, each on a stream and in a workspace of its own
+    // (one that is done leaves its SMs to the next), or, where the device has no
+    // room for all workspaces, one after the other in one of them.
+    bool apart = groups.size() > 1;
+    if (apart && ensure_ws(c0, ws)) apart = false;
+    if (!apart && (rc = ensure_ws(c0, most))) return rc;
+    for (size_t i = c0->side.size(); apart && i + 1 < groups.size(); ++i) {
+        cudaStream_t s = nullptr;
+        CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        c0->side.push_back(s);
+    }
+    std::vector<unsigned char> host(bytes, 0);  // the inputs as on the device, then the results
+    memcpy(host.data(), energies, sizeof(double) * nE);
+    for (const BatchGroup &g : groups) {
+        for (size_t m = 0; m < g.members.size(); ++m) ((Geo *)(host.data() + g.geo_at))[m] = make_geo(ctxs[g.members[m]]);
+        for (size_t q = 0; q < g.order.size(); ++q) ((BatchJob *)(host.data() + g.jobs_at))[q] = g.jobs[g.order[q]];
+    }
+    unsigned char *dev = nullptr;
+    if (cudaMalloc(&dev, bytes) != cudaSuccess) { cudaGetLastError(); return NEGF_ERR_NOMEM; }
+    float ms = 0.f;
+    if (cudaMemcpyAsync(dev, host.data(), in_bytes, cudaMemcpyHostToDevice, c0->stream) || cudaEventRecord(c0->ev0, c0->stream))
+        rc = NEGF_ERR_CUDA;
+    for (size_t i = 0; i < groups.size() && !rc; ++i) {
+        const BatchGroup &g = groups[i];
+        cudaStream_t st = apart && i > 0 ? c0->side[i - 1] : c0->stream;
+        if (st != c0->stream && cudaStreamWaitEvent(st, c0->ev0, 0)) rc = NEGF_ERR_CUDA;
+        if (!rc)
+            rc = launch_batch(g.k, g.sh, (const Geo *)(dev + g.geo_at), (const BatchJob *)(dev + g.jobs_at), (int)g.jobs.size(),
+                              (const double *)dev, (double2 *)((unsigned char *)c0->d_ws + (apart ? g.ws_at : 0)), g.k.ws,
+                              (double *)(dev + g.tau_at), (int *)(dev + g.info_at), (int *)(dev + g.counter_at), st);
+    }
+    // ev1 marks the end of each side stream in turn, waited for by the first one
+    for (size_t i = 1; apart && i < groups.size(); ++i)
+        if (cudaEventRecord(c0->ev1, c0->side[i - 1]) || cudaStreamWaitEvent(c0->stream, c0->ev1, 0)) rc = NEGF_ERR_CUDA;
+    if (!rc && (cudaEventRecord(c0->ev1, c0->stream) ||
+                cudaMemcpyAsync(host.data() + in_bytes, dev + in_bytes, bytes - in_bytes, cudaMemcpyDeviceToHost, c0->stream) ||
+                cudaStreamSynchronize(c0->stream) || cudaEventElapsedTime(&ms, c0->ev0, c0->ev1)))
+        rc = NEGF_ERR_CUDA;
+    if (rc) cudaDeviceSynchronize();
+    cudaFree(dev);
     if (rc) return rc;
-    fill_stats(stats, info_all, ms_all);
-    return first_info(info_all);
+    std::vector<int> info;
+    for (const BatchGroup &g : groups) {
+        const double *t = (const double *)(host.data() + g.tau_at);
+        const int *in = (const int *)(host.data() + g.info_at);
+        info.insert(info.end(), in, in + g.jobs.size());
+        // tau[p][e] = sum_k w_k tau(p, e, k), summed in k order (negf.f90:172)
+        std::vector<double> per(g.jobs.size());
+        for (size_t q = 0; q < g.order.size(); ++q) per[g.order[q]] = t[q];
+        for (size_t q = 0; q < g.jobs.size(); ++q) {
+            const int p = g.members[g.jobs[q].prob];
+            tau[(size_t)p * nE + g.jobs[q].ie] += per[q] * ctxs[p]->kpt[3 * g.jobs[q].ik + 2];
+        }
+    }
+    fill_stats(stats, info, ms);
+    return first_info(info);
 }
 
 // ------------------------------------------------------ real-space outputs

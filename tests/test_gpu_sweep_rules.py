@@ -197,3 +197,68 @@ def test_real_space_density_of_the_longest_basis():
     with Engine(nx, ny, np.zeros((4 * mx + 1, 1, 2), complex), 1.0, 1.0, 1.0, 0.0, 0.0, 1e-6, [[0, 0, 1]]) as eng:
         got = eng.dm_real(G, 2 * mx + 3, 1, 1.0, 1.0, 2.0)
     assert np.max(np.abs(got - ref.imag)) <= 1e-12 * N
+
+
+# the kernels of a batch run side by side: bases of every kernel, jobs above and below the number of slots
+@pytest.mark.parametrize("nE", [3, 60])
+def test_batch_of_every_kernel(oracle, nE):
+    probs = [cut_problem(oracle, N, nz) for N, nz in ((20, 4), (40, 3), (72, 3), (150, 2), (256, 2), (260, 2), (290, 2))]
+    E = np.linspace(0.05, 0.2, nE) * probs[3][2]
+    check = slice(None) if nE < 10 else slice(0, nE, 19)
+    bad = E.copy()
+    bad[1] = np.nan
+    engines = [Engine(*p[0]) for p in probs]
+    try:
+        tau, info, stats = transmission_batch(engines, E)
+        tau_bad, info_bad, stats_bad = transmission_batch(engines, bad)
+        turned, _, _ = transmission_batch(engines[::-1], E)
+    finally:
+        for e in engines:
+            e.close()
+    assert info == 0 and stats.n_jobs == nE * len(probs) and stats.n_singular == 0
+    assert info_bad > 0 and stats_bad.n_singular == len(probs)
+    assert (turned[::-1] == tau).all()
+    keep = np.arange(nE) != 1
+    for p, t, b in zip(probs, tau, tau_bad):
+        ref, _ = oracle.transmission_jobs(p[1], E[check], nthreads=8)
+        np.testing.assert_allclose(t[check], ref, rtol=RTOL, atol=ATOL)
+        assert (b[keep] == t[keep]).all()
+
+
+def test_one_wide_basis_does_not_slow_a_batch(oracle):
+    """1800 sweeps of N = 221 fill the chip two to an SM; a base above 256 beside them leaves them there."""
+    a = cut_problem(oracle, 221, 8)[0]
+    w = cut_problem(oracle, 260, 2)[0]
+    E = np.linspace(0.01, 0.2, 150) * 1e-4
+    engines = [Engine(*a) for _ in range(12)] + [Engine(*w)]
+    try:
+        def ms(which):
+            return min(transmission_batch(which, E)[2].device_ms for _ in range(3))
+        # the 300 slices of N = 260 are 1.04 times the work; in panels those of N = 221 took 1.19 times as long
+        assert ms(engines) <= 1.12 * ms(engines[:-1])
+    finally:
+        for e in engines:
+            e.close()
+
+
+# workspaces of 58 MB (N = 300) and 15 MB (N = 221): side by side, and one after the other where 66 MB are free
+def test_batch_in_little_memory(oracle):
+    import torch
+    probs = [cut_problem(oracle, N, 2) for N in (300, 221)]
+    E = np.linspace(0.05, 0.2, 10) * probs[0][2]
+    engines = [Engine(*p[0]) for p in probs]
+    other = [Engine(*p[0]) for p in probs]
+    try:
+        ref, _, _ = transmission_batch(engines, E)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - 66000000, dtype=torch.uint8, device="cuda")
+        try:
+            tau, info, _ = transmission_batch(other, E)
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+    finally:
+        for e in engines + other:
+            e.close()
+    assert info == 0 and (tau == ref).all()
