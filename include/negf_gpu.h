@@ -197,10 +197,11 @@ int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, const double *e
 /* Transmission kernel variants (no reference counterpart: the reference has
  * one LAPACK path, math_kernel.f90:8-42): panel width x rows per thread x
  * CTAs per SM, 0 = 16 x 1 x 2 (N <= 256), 1 = 16 x 2 x 1 (N <= 512),
- * 2 = 8 x 4 x 1 (N <= 1024), 3 = the on-chip family (N <= 256): the block in
+ * 2 = 8 x 4 x 1 (N <= 1024), 3 = the on-chip family (N <= 272): the block in
  * registers up to 72 plane waves; above, panels in registers with a cluster of
- * CTAs per job for few jobs, else 8 x 1 x 2.  By default the variant follows
- * N: 3 up to 272, then 1, then 2.
+ * CTAs per job for few jobs (above 256 for any number) whose open channels the
+ * panels have room for, else 8 x 1 x 2 (above 256 16 x 2 x 1).  By default the
+ * variant follows N: 3 up to 272, then 1, then 2.
  * negf_set_variant forces one for this context's negf_transmission[_device]
  * and negf_transmission_batch calls (-1 = back to the default;
  * NEGF_ERR_UNSUPPORTED if it cannot hold N).  negf_autotune times every

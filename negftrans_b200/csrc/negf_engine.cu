@@ -401,7 +401,7 @@ Variant pick_variant(int N) {
 }
 bool variant_fits(int v, int N) {
     return (v == V16x1 && N <= NT) || (v == V16x2 && N <= 2 * NT) || (v == V8x4 && N <= 4 * NT) ||
-           (v == VCHIP && N <= NT);
+           (v == VCHIP && N <= PNMAX);
 }
 // Default variant of the transmission kernels: variant 3 up to PNMAX plane waves
 // (sweep_kernel says which kernel that is), then the narrowest that holds N.  The slab kernels keep pick_variant:

@@ -8,6 +8,7 @@ import pytest
 
 from negftrans_b200 import prepare as P
 from negftrans_b200 import workloads as W
+from negftrans_b200._lib import NEGF_ERR_UNSUPPORTED, NegfError
 from negftrans_b200.negf import Engine, GreensFunction_tri_solver, transmission_batch
 
 pytestmark = pytest.mark.gpu
@@ -262,3 +263,25 @@ def test_batch_in_little_memory(oracle):
         for e in engines + other:
             e.close()
     assert info == 0 and (tau == ref).all()
+
+
+@pytest.mark.parametrize("N", [257, 272])
+def test_the_autotuner_times_the_default_kernel(oracle, N):
+    args, op, kmax = cut_problem(oracle, N, nz=3)
+    E = np.linspace(0.02, 0.12, 20) * kmax
+    ref, _ = oracle.transmission_jobs(op, E[::7], nthreads=8)
+    with Engine(*args) as eng:
+        default, _ = eng.transmission(E)
+        ms = min((eng.transmission(E), eng.last_stats.device_ms)[1] for _ in range(3))
+        eng.set_variant(3)
+        forced, _ = eng.transmission(E)
+        assert (forced == default).all()
+        np.testing.assert_allclose(forced[::7], ref, rtol=RTOL, atol=ATOL)
+        v, rates = eng.autotune(E)
+        assert rates[0] == 0 and (rates[1:] > 0).all() and rates[v] == rates.max()
+        eng.transmission(E)
+        # a tuned call is no slower than an untuned one: 16 x 2 x 1 takes 2.4 times as long here
+        assert eng.last_stats.device_ms <= 1.2 * ms
+    with Engine(*cut_problem(oracle, 273, nz=2)[0]) as eng, pytest.raises(NegfError) as exc:
+        eng.set_variant(3)
+    assert exc.value.code == NEGF_ERR_UNSUPPORTED
