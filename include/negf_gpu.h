@@ -200,8 +200,8 @@ int negf_transmission_batch(negf_ctx *const *ctxs, int32_t nctx, const double *e
  * 2 = 8 x 4 x 1 (N <= 1024), 3 = the on-chip family (N <= 272): the block in
  * registers up to 72 plane waves; above, panels in registers with a cluster of
  * CTAs per job for few jobs (above 256 for any number) whose open channels the
- * panels have room for, else 8 x 1 x 2 (above 256 16 x 2 x 1).  By default the
- * variant follows N: 3 up to 272, then 1, then 2.
+ * panels have room for, else 8 x 1 x 2, 8 x 1 x 1 for at most one job per SM
+ * (above 256 16 x 2 x 1).  By default the variant follows N: 3 up to 272, then 1, then 2.
  * negf_set_variant forces one for this context's negf_transmission[_device]
  * and negf_transmission_batch calls (-1 = back to the default;
  * NEGF_ERR_UNSUPPORTED if it cannot hold N).  negf_autotune times every

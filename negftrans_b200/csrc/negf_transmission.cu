@@ -10,7 +10,7 @@ namespace {
 // k-point ik) of problem g, in the workspace A0 (four ld x N blocks).  The
 // basis must already be in s.nx / s.ny.  Returns tau in *tau (thread 0) and
 // the LAPACK-style info.
-template <int NB, int RPT>
+template <int NB, int RPT, bool WIDE>
 __device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, double2 *A0, double *tau) {
     const int N = g.N, ld = g.ld, Nz = g.Nz;
     double2 *A1 = A0 + (size_t)ld * N;
@@ -26,7 +26,7 @@ __device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, d
     // generator_r(N_z-1) = inv(D_Nz)          math_kernel.f90:82
     form_block(cur, g, s, Nz - 1, E, ik, nullptr, nullptr);
     __syncthreads();
-    int info = gj_invert<NB, RPT>(cur, N, ld, s);
+    int info = gj_invert<NB, RPT, WIDE>(cur, N, ld, s);
     unpermute_rows(P, ld, cur, ld, N, nr, s);
     __syncthreads();
     // generator_r(m) = inv(D_{m+1} - generator_r(m+1)), with the rows of the
@@ -36,7 +36,7 @@ __device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, d
     for (int m = Nz - 3; m >= 0; --m) {
         form_block(oth, g, s, m + 1, E, ik, cur, nullptr);
         __syncthreads();
-        const int r = gj_invert<NB, RPT>(oth, N, ld, s);
+        const int r = gj_invert<NB, RPT, WIDE>(oth, N, ld, s);
         if (r && !info) info = r;
         GemmArgs ga{Pn, ld, P, ld, s.iprow, oth, ld, s.iprow, nr, N, N, nullptr};
         cta_gemm(ga, s, GEMM_STORE, g.delta);
@@ -47,7 +47,7 @@ __device__ int transmission_job(const Geo &g, const Smem &s, double e, int ik, d
     // G_11 = inv(D_1 - generator_r(1))          math_kernel.f90:113-118
     form_block(oth, g, s, 0, E, ik, cur, nullptr);
     __syncthreads();
-    const int r = gj_invert<NB, RPT>(oth, N, ld, s);
+    const int r = gj_invert<NB, RPT, WIDE>(oth, N, ld, s);
     if (r && !info) info = r;
     // tau = sum_ij gamma_L,i gamma_R,j |2 dz^2 G_{Nz,1}(i,j)|^2   grid.f90:362-383
     GemmArgs ga{nullptr, 0, P, ld, s.iprow, oth, ld, s.iprow, nr, N, N, s.rows};
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(NT, MINB)
         // job -> (energy, k-point), energy fastest: negf.f90:131-133
         const int ie = job % nE, ik = job / nE;
         double t = 0.0;
-        const int info = transmission_job<NB, RPT>(g, s, energies[ie], ik, A0, &t);
+        const int info = transmission_job<NB, RPT, MINB == 1>(g, s, energies[ie], ik, A0, &t);
         if (threadIdx.x == 0) {
             tau_jobs[job] = t;
             if (info_jobs) info_jobs[job] = info;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(NT, MINB)
         for (int i = threadIdx.x; i < g.N; i += NT) { s.nx[i] = g.nx[i]; s.ny[i] = g.ny[i]; }
         __syncthreads();
         double t = 0.0;
-        const int info = transmission_job<NB, RPT>(g, s, energies[jb.ie], jb.ik, A0, &t);
+        const int info = transmission_job<NB, RPT, MINB == 1>(g, s, energies[jb.ie], jb.ik, A0, &t);
         if (threadIdx.x == 0) {
             tau_jobs[q] = t;
             info_jobs[q] = info;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(NT, MINB)
 template <int NB, int RPT, int MINB>
 SweepKernel make(int N) {
     return SweepKernel{(const void *)k_transmission<NB, RPT, MINB>, (const void *)k_transmission_batch<NB, RPT, MINB>,
-                       NT, smem_bytes<NB, RPT>(N), 4 * (size_t)round_up(N, 8) * N};
+                       NT, smem_bytes<NB, RPT, MINB == 1>(N), 4 * (size_t)round_up(N, 8) * N};
 }
 
 }  // namespace
@@ -128,7 +128,8 @@ SweepKernel sweep_kernel(Variant v, int N, int share, int open) {
         case VCHIP:
             if (N <= RNMAX) return register_kernel(N);
             if ((share >= 2 || N > NT) && open <= panel_channels(N) * (share >= 8 ? 2 : 1)) return panel_kernel(N);
-            return N > NT ? make<16, 2, 1>(N) : make<8, 1, 2>(N);
+            if (N > NT) return make<16, 2, 1>(N);
+            return share >= 1 ? make<8, 1, 1>(N) : make<8, 1, 2>(N);
         default: return SweepKernel{};
     }
 }

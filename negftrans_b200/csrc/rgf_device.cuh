@@ -160,12 +160,13 @@ struct Smem {
 
 __host__ __device__ inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-template <int NB, int RPT>
+// WIDE: one CTA per SM, trailing_update_wide.
+template <int NB, int RPT, bool WIDE = (RPT > 1)>
 __host__ __device__ inline size_t smem_bytes(int N) {
     int ldw = round_up(N, CM);
     size_t big = (size_t)NB * ldw + (size_t)NB * NB;         // sub-panel a + 16x16 block
     // rank-32 update: gathered rows + 2 x 32 rows of W, or (wide) two of each tile
-    size_t trail = RPT > 1 ? 2 * 32 * (size_t)(BP + AP) : 32 * (size_t)(BP + 2 * TP);
+    size_t trail = WIDE ? 2 * 32 * (size_t)(BP + AP) : 32 * (size_t)(BP + 2 * TP);
     size_t gemm = 2 * (size_t)KC * (AP + BP);
     if (trail > big) big = trail;
     if (gemm > big) big = gemm;
@@ -851,7 +852,7 @@ __device__ inline void factor_subpanel(double2 (&w)[RPT][NB], int kb, int nbe, u
 // On return s.prow/s.iprow hold the permutations (inv(A)(r,c) =
 // A(prow[r], iprow[c])).  Returns the LAPACK-style info (1-based column of
 // the first zero pivot, 0 if none); identical in every thread.
-template <int NB, int RPT>
+template <int NB, int RPT, bool WIDE>
 __device__ int gj_invert_pair(double2 *__restrict__ A, int N, int ld, const Smem &s) {
     const int tid = threadIdx.x;
     const int ldw = s.ldw;
@@ -953,7 +954,7 @@ __device__ int gj_invert_pair(double2 *__restrict__ A, int N, int ld, const Smem
         }
         __syncthreads();
         if (nbt < N) {
-            if constexpr (RPT > 1) trailing_update_wide<2 * NB>(A, N, ld, k0, nbt, s);
+            if constexpr (WIDE) trailing_update_wide<2 * NB>(A, N, ld, k0, nbt, s);
             else trailing_update<2 * NB>(A, N, ld, k0, nbt, s);
         }
         __syncthreads();
@@ -973,7 +974,7 @@ __device__ int gj_invert_pair(double2 *__restrict__ A, int N, int ld, const Smem
 // apply its steps to the earlier columns, W_{<p} = mask_p(W_{<p}) +
 // W_p W_{<p}(P_p); the trailing update then applies the whole panel at once,
 // the single-panel formula of trailing_update with W = A(:, panel).
-template <int NB, int RPT, int P>
+template <int NB, int RPT, int P, bool WIDE>
 __device__ int gj_invert_multi(double2 *__restrict__ A, int N, int ld, const Smem &s) {
     const int tid = threadIdx.x;
     const double2 zero = make_double2(0.0, 0.0);
@@ -1058,7 +1059,7 @@ __device__ int gj_invert_multi(double2 *__restrict__ A, int N, int ld, const Sme
             __syncthreads();
         }
         if (nbt < N) {
-            if constexpr (RPT > 1) trailing_update_wide<P * NB>(A, N, ld, k0, nbt, s);
+            if constexpr (WIDE) trailing_update_wide<P * NB>(A, N, ld, k0, nbt, s);
             else trailing_update<P * NB>(A, N, ld, k0, nbt, s);
         }
         __syncthreads();
@@ -1073,10 +1074,10 @@ __device__ int gj_invert_multi(double2 *__restrict__ A, int N, int ld, const Sme
 // The inverse used by the kernels: 16-column sub-panels in pairs through
 // shared memory; 8-column sub-panels (the large-N variant) four per panel
 // through A, so that every variant applies rank-32 trailing updates.
-template <int NB, int RPT>
+template <int NB, int RPT, bool WIDE = (RPT > 1)>
 __device__ int gj_invert(double2 *__restrict__ A, int N, int ld, const Smem &s) {
-    if constexpr (NB == 8) return gj_invert_multi<8, RPT, 4>(A, N, ld, s);
-    else return gj_invert_pair<NB, RPT>(A, N, ld, s);
+    if constexpr (NB == 8) return gj_invert_multi<8, RPT, 4, WIDE>(A, N, ld, s);
+    else return gj_invert_pair<NB, RPT, WIDE>(A, N, ld, s);
 }
 
 }  // namespace negf

@@ -43,7 +43,11 @@ enum Variant { V16x1 = 0, V16x2 = 1, V8x4 = 2, VCHIP = 3, VNONE = 4 };
 // of eight) or N > 256 (148 jobs of N = 257, N_z = 6, 14.5 ms in 16 x 2 x 1, which
 // takes a whole SM as well, 10.7 in panels; N = 272 15.2 and 12.8); otherwise
 // 8 x 1 x 2, whose two jobs per SM cover each other's pivots (N = 221: 840 us of
-// an SM per slice and job, the panel kernel alone on an SM 1160).
+// an SM per slice and job, the panel kernel alone on an SM 1000), or 8 x 1 x 1
+// where every job has an SM to itself: the pipelined 64 x 64 tiles of the
+// one-CTA variants (148 jobs of N = 128, 221, 256, N_z = 8, 2.76 -> 2.31, 9.3 -> 8.0,
+// 13.6 -> 11.1 ms; 32 x 64 tiles alone on an SM were up to 4 % slower than unpipelined
+// ones).
 //
 // A block of the panel kernel has room for panel_channels(N) channels; more
 // take another sweep each time, where the other kernels only carry a wider

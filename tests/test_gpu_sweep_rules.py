@@ -285,3 +285,54 @@ def test_the_autotuner_times_the_default_kernel(oracle, N):
     with Engine(*cut_problem(oracle, 273, nz=2)[0]) as eng, pytest.raises(NegfError) as exc:
         eng.set_variant(3)
     assert exc.value.code == NEGF_ERR_UNSUPPORTED
+
+
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+# above one job per two SMs: one CTA per SM (8 x 1 x 1), two (8 x 1 x 2), and more jobs than places; panels above 256
+@pytest.mark.parametrize("N", [73, 96, 97, 129, 192, 193, 221, 255, 256, 257, 272])
+def test_many_jobs_of_middle_bases(oracle, N):
+    args, op, kmax = cut_problem(oracle, N, nz=2)
+    with Engine(*args) as eng:
+        for nE in (sms() // 2 + 1, sms() + 1, 2 * sms() + 3):
+            E = np.concatenate([[-1e-6], np.linspace(0.01, 0.15, nE - 1) * kmax])
+            check = [0, 1, nE // 2, nE - 2, nE - 1]
+            ref, _ = oracle.transmission_jobs(op, E[check], nthreads=8)
+            tau, info = eng.transmission(E)
+            both, _, stats = transmission_batch([eng], E)
+            assert info == 0 and stats.n_jobs == nE
+            np.testing.assert_allclose(tau[check], ref, rtol=RTOL, atol=ATOL)
+            assert (both[0] == tau).all()
+
+
+# remainders of the 32-column panels and of the 32- and 64-row tiles
+@pytest.mark.parametrize("N", [65, 97, 100, 191, 225, 256])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+def test_every_variant_beyond_one_panel(oracle, N, variant):
+    args, op, kmax = cut_problem(oracle, N, nz=3)
+    E = np.linspace(0.05, 1.2, 4) * kmax
+    ref, _ = oracle.transmission_jobs(op, E, nthreads=8)
+    with Engine(*args) as eng:
+        eng.set_variant(variant)
+        tau, info = eng.transmission(E)
+    assert info == 0
+    np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
+
+
+def test_batch_of_many_middle_bases(oracle):
+    """More sweeps than places, all of 73 to 256 plane waves: two on an SM, taken from one counter."""
+    probs = [cut_problem(oracle, N, nz) for N, nz in ((73, 3), (256, 2), (129, 2), (221, 2))]
+    E = np.linspace(0.02, 0.3, sms()) * probs[0][2]
+    engines = [Engine(*p[0]) for p in probs]
+    try:
+        tau, info, stats = transmission_batch(engines, E)
+    finally:
+        for e in engines:
+            e.close()
+    assert info == 0 and stats.n_jobs == 4 * len(E)
+    for p, t in zip(probs, tau):
+        ref, _ = oracle.transmission_jobs(p[1], E[::49], nthreads=8)
+        np.testing.assert_allclose(t[::49], ref, rtol=RTOL, atol=ATOL)
