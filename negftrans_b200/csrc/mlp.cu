@@ -374,7 +374,7 @@ int negf_mlp_create(int32_t n_layers, const int32_t *widths, int32_t max_batch, 
     alloc(&m->ones, (size_t)max_batch);
     if (ok) {
         std::vector<float> one((size_t)max_batch, 1.0f);
-        ok = cudaMemcpy(m->ones, one.data(), sizeof(float) * max_batch, cudaMemcpyHostToDevice) == cudaSuccess;
+        ok = cudaMemcpyAsync(m->ones, one.data(), sizeof(float) * max_batch, cudaMemcpyHostToDevice, m->st) == cudaSuccess;
     }
     if (ok) ok = cudaMalloc(&m->loss, sizeof(double)) == cudaSuccess;
     if (ok) ok = cudaMemsetAsync(m->p, 0, sizeof(float) * m->np, m->st) == cudaSuccess &&

@@ -768,12 +768,16 @@ int negf_ctx_create(const negf_problem *p, int32_t device, negf_ctx **out) {
     CKC(cudaMalloc(&c->d_ay, sizeof(double) * ay.size()));
     CKC(cudaMalloc(&c->d_kw, sizeof(double) * kw.size()));
     CKC(cudaMalloc(&c->d_open, sizeof(int)));
-    CKC(cudaMemcpy(c->d_vhat, p->vhat, sizeof(double2) * nv, cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_nx, p->nx, sizeof(int) * p->N, cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_ny, p->ny, sizeof(int) * p->N, cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_ax, ax.data(), sizeof(double) * ax.size(), cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_ay, ay.data(), sizeof(double) * ay.size(), cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_kw, kw.data(), sizeof(double) * kw.size(), cudaMemcpyHostToDevice));
+    // on the context's stream and waited for: a copy from pageable memory may
+    // return before it is done, and later calls run on streams that do not wait
+    // for the default one
+    CKC(cudaMemcpyAsync(c->d_vhat, p->vhat, sizeof(double2) * nv, cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_nx, p->nx, sizeof(int) * p->N, cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_ny, p->ny, sizeof(int) * p->N, cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_ax, ax.data(), sizeof(double) * ax.size(), cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_ay, ay.data(), sizeof(double) * ay.size(), cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_kw, kw.data(), sizeof(double) * kw.size(), cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaStreamSynchronize(c->stream));
 #undef CKC
     *out = c;
     return NEGF_OK;

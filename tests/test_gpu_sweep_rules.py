@@ -336,3 +336,15 @@ def test_batch_of_many_middle_bases(oracle):
     for p, t in zip(probs, tau):
         ref, _ = oracle.transmission_jobs(p[1], E[::49], nthreads=8)
         np.testing.assert_allclose(t[::49], ref, rtol=RTOL, atol=ATOL)
+
+
+def test_context_has_its_inputs_when_it_is_made(oracle):
+    """7 MB of V table, another one at each context, used at once; the sweep starts at its last slice."""
+    for seed in (1, 2, 3):
+        args, op, kmax = cut_problem(oracle, 20, nz=1500, grid=32, seed=seed)
+        E = np.array([4.0, 5.0]) * kmax
+        ref, _ = oracle.transmission_jobs(op, E, nthreads=4)
+        with Engine(*args) as eng:
+            tau, info = eng.transmission(E)
+        assert info == 0
+        np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
