@@ -40,6 +40,22 @@ struct negf_ctx {
     double2 *d_voff = nullptr;
 };
 
+// Opts a kernel into all the dynamic shared memory it can have.  The limit is one
+// per kernel and process, so it is always the same value: with each call's own
+// size, another thread's smaller call between this one's opt-in and its launch
+// would make the launch fail.
+template <typename F>
+inline cudaError_t allow_smem(F *kernel) {
+    const void *fn = (const void *)kernel;
+    cudaFuncAttributes a;
+    int dev = 0, most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&a, fn);
+    if (!e) e = cudaGetDevice(&dev);
+    if (!e) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (!e) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    return e;
+}
+
 // FP64 sweeps of the listed jobs (energy index ie[q] into h_E and d_E, k-point
 // ik[q]) of context c through the batch kernel: h_tau[q] the unweighted tau of
 // job q, h_info[q] its info; *ms the device time.  Synchronous on c->stream.

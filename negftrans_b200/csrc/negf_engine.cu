@@ -413,7 +413,7 @@ Variant ctx_variant(const negf_ctx *c) {
 }
 // Opts a kernel into its dynamic shared memory; *occ = its resident CTAs per SM.
 int prep_kernel(const void *fn, int threads, size_t smem, int *occ) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem(fn));
     int o = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, threads, smem));
     *occ = o > 0 ? o : 1;
@@ -1495,7 +1495,7 @@ int launch_ptor(negf_ctx *c, const double2 *d_G, int nslices, int Nx, int Ny, do
     if (2 * mx >= Nx || 2 * my >= Ny) return NEGF_ERR_ARG;  // index nx+Nx/2 must fit (grid.f90:92-94)
     if (ptor_smem(mx, my, Nx, Ny) > 200 * 1024) return NEGF_ERR_UNSUPPORTED;
     const size_t smem = ptor_smem(mx, my, Nx, Ny) + ptor_lists(c->N, mx, my);
-    CK(cudaFuncSetAttribute(k_ptor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem(k_ptor));
     k_ptor<<<nslices, PT_THREADS, smem, st>>>(d_G, c->N, ldg ? ldg : c->N, gstride ? gstride : (size_t)c->N * c->N,
                                               c->d_nx, c->d_ny, mx, my, Nx, Ny, scale, d_dens, d_cdiag);
     CK(cudaGetLastError());
@@ -1556,7 +1556,7 @@ extern "C" int negf_vhat_gpu(const double *vreal, int32_t Nx, int32_t Ny, int32_
     if (!rc && (cudaMemcpyAsync(d_v, vreal, sizeof(double) * nv, cudaMemcpyHostToDevice, st) != cudaSuccess ||
                 cudaMemcpyAsync(d_t, tx.data(), sizeof(double2) * Nx, cudaMemcpyHostToDevice, st) != cudaSuccess ||
                 cudaMemcpyAsync(d_t + Nx, ty.data(), sizeof(double2) * Ny, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-                cudaFuncSetAttribute(k_vhat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess))
+                allow_smem(k_vhat) != cudaSuccess))
         rc = NEGF_ERR_CUDA;
     if (!rc) {
         k_vhat<<<Nz, VH_THREADS, smem, st>>>(d_v, Nx, Ny, ngx, ngy, d_t, d_t + Nx, d_h);

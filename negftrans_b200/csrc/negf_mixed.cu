@@ -2100,7 +2100,7 @@ extern "C" int negf_tc_product_check(const float *d_W, int32_t ldw, const float 
         return NEGF_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t smem = gj_smem_bytes(32) + tile_smem_bytes();
-    CKM(cudaFuncSetAttribute(k_tc_product_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CKM(allow_smem(k_tc_product_check));
     int *d_status = nullptr;
     CKM(cudaMalloc(&d_status, sizeof(int)));
     CKM(cudaMemsetAsync(d_status, 0, sizeof(int), st));
@@ -2137,7 +2137,7 @@ extern "C" int negf_tc_inverse_check(const float *d_A, int32_t N, int32_t nmat, 
         cudaFree(pscr);
         return NEGF_ERR_CUDA;
     }
-    CKM(cudaFuncSetAttribute(k_tc_inverse_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CKM(allow_smem(k_tc_inverse_check));
     k_tc_inverse_check<<<nmat, NT, smem, st>>>(work, N, ld, (float2 *)d_out, d_info, d_status, pscr, tm);
     CKM(cudaGetLastError());
     int h = 0;
@@ -2191,12 +2191,6 @@ cudaError_t launch_pass(const MixedArgs &a, int nw, int cpj, size_t smem, cudaSt
     lc.attrs = la;
     lc.numAttrs = 1;
     return cudaLaunchKernelEx(&lc, k_mixed_pass, a, mode, it, last);
-}
-
-template <typename K>
-int set_smem(K kern, size_t bytes) {
-    CKM(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return 0;
 }
 
 }  // namespace
@@ -2289,7 +2283,7 @@ int negf_internal_mixed(negf_ctx *c, const double *h_E, const double *d_E, int n
         while (pa > PA_MIN && pass_smem_bytes(N, ncap, pa) + 1024 > (size_t)smem_optin) --pa;
         if (sm_sweep > (size_t)smem_optin || pass_smem_bytes(N, ncap, pa) + 1024 > (size_t)smem_optin) W = 0;
         if (cpj == 2 && W >= 1) {
-            CKM(cudaFuncSetAttribute(k_mixed_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_sweep));
+            CKM(allow_smem(k_mixed_sweep));
             cudaLaunchConfig_t qc = {};
             cudaLaunchAttribute qa[1];
             qa[0].id = cudaLaunchAttributeClusterDimension;
@@ -2343,9 +2337,7 @@ int negf_internal_mixed(negf_ctx *c, const double *h_E, const double *d_E, int n
             const size_t sm_pass = pass_smem_bytes(N, ncap, pa);
             a.pa = pa;
             const size_t sm_res = (size_t)2 * negf::KC * (negf::AP + negf::BP) * 16 + job_smem_bytes(N);
-            rc = set_smem(k_mixed_sweep, sm_sweep);
-            if (!rc) rc = set_smem(k_mixed_pass, sm_pass);
-            if (!rc) rc = set_smem(k_mixed_residual, sm_res);
+            if (allow_smem(k_mixed_sweep) || allow_smem(k_mixed_pass) || allow_smem(k_mixed_residual)) rc = NEGF_ERR_CUDA;
             if (rc) return rc;
             CUtensorMap tmC;
             if (!c_tile_map(&tmC, a.scratch, N, c->ld, 2, (size_t)N * c->ld * 8, W, L.scratch_bytes))

@@ -348,3 +348,54 @@ def test_context_has_its_inputs_when_it_is_made(oracle):
             tau, info = eng.transmission(E)
         assert info == 0
         np.testing.assert_allclose(tau, ref, rtol=RTOL, atol=ATOL)
+
+
+def test_contexts_in_two_threads(oracle):
+    """Calls of different bases in the same kernels, 200 in each of three threads."""
+    import threading
+    probs = [cut_problem(oracle, N, 2) for N in (80, 160, 256)]
+    E = [np.linspace(0.05, 0.15, 3) * p[2] for p in probs]
+    ref = [oracle.transmission_jobs(p[1], e, nthreads=8)[0] for p, e in zip(probs, E)]
+    seen = [None] * len(probs)
+
+    def work(i):
+        try:
+            with Engine(*probs[i][0]) as eng:
+                for _ in range(200):
+                    tau, info = eng.transmission(E[i])
+                    assert info == 0
+                    np.testing.assert_allclose(tau, ref[i], rtol=RTOL, atol=ATOL)
+                seen[i] = "done"
+        except Exception as e:
+            seen[i] = repr(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(probs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == ["done"] * len(probs)
+
+
+@pytest.mark.parametrize("N,nE", [(69, 3), (221, 3), (221, 80), (272, 20)])
+def test_transmission_in_a_graph(oracle, N, nE):
+    """The device entry under stream capture, one kernel or two, replayed on other energies."""
+    import torch
+    args, op, kmax = cut_problem(oracle, N, nz=2)
+    with Engine(*args) as eng:
+        dE = torch.linspace(0.05, 0.15, nE, dtype=torch.float64, device="cuda") * kmax
+        dt = torch.zeros(nE, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        eng.transmission_device(dE.data_ptr(), nE, dt.data_ptr())  # grows the workspace
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            eng.transmission_device(dE.data_ptr(), nE, dt.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        for top in (0.12, 1.2):
+            E = np.linspace(0.05, top, nE) * kmax
+            dE.copy_(torch.tensor(E))
+            graph.replay()
+            torch.cuda.synchronize()
+            ref, _ = oracle.transmission_jobs(op, E[::7], nthreads=8)
+            np.testing.assert_allclose(dt.cpu().numpy()[::7], ref, rtol=RTOL, atol=ATOL)
+        del graph
