@@ -1,14 +1,16 @@
-// negf_engine.cu -- kernels and C ABI of the FP64 RGF engine (sm_100a).
+// negf_engine.cu -- host code and C ABI of the FP64 RGF engine (sm_100a).
 //
 // Replaces the per-job drivers of src/negf.f90 and the solver of
-// src/math_kernel.f90.  Three kernels carry the hot path:
-//   k_transmission  F-mode streaming sweep + transmission epilogue, one CTA
-//                   per (E,k) job, O(N^2) state per job (negf.f90:115-174)
-//   k_rgf_slab      sweeps that keep every generator block, for the diagonal
-//                   (density, LDOS) and first/last-column (tri_solve) blocks
-//                   (negf.f90:9-113, 176-236; math_kernel.f90:44-165)
+// src/math_kernel.f90.  The sweeps are kernels of other files, launched from
+// here by the descriptions of sweep_kernels.h: transmission (negf.f90:115-174)
+// in negf_register.cu, negf_panel.cu and negf_transmission.cu; the sweeps that
+// keep every generator block, for density, LDOS and tri_solve (negf.f90:9-113,
+// 176-236; math_kernel.f90:44-165), in negf_register_slab.cu and negf_slab.cu.
+// The kernels here sum, check and transform their results:
 //   k_accumulate    weighted sum of the diagonal blocks over the jobs of a
 //                   chunk (the accumulation loops of negf.f90:86-111,226-234)
+//   k_ptor, k_vhat  plane waves to real space and back
+//   k_most_open     open channels of a call, which the choice of kernel needs
 #include <cuda_runtime.h>
 #include <math_constants.h>
 

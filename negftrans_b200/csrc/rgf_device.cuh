@@ -6,8 +6,9 @@
 // from HBM: D_k = 2*dz^2*((E+i*eta)I - H_k) - 2I (grid.f90:236-333) is
 // generated from the V(G-G') table while the previous inverse is subtracted.
 // Inverses use a blocked Gauss-Jordan elimination with implicit partial
-// pivoting (the pivot choice of LAPACK zgetf2: largest |re|+|im| among the
-// rows not yet used), whose panel lives in registers; the rank-NB trailing
+// pivoting (LAPACK zgetf2's rule, the largest |re|+|im| among the rows not yet
+// used, but magnitudes that agree to 17 bits tie: the pivot is the largest up
+// to 1 part in 2^17), whose panel lives in registers; the rank-NB trailing
 // update and the chain products are complex FP64 GEMMs tiled through shared
 // memory.  The raw Gauss-Jordan result R satisfies
 //     inv(M)(r, c) = R(prow[r], iprow[c])
@@ -765,8 +766,9 @@ __device__ inline int warp_pivot(const double2 (&f)[RPT], unsigned used, int buf
 
 // Gauss-Jordan elimination of the columns [kb, kb+nbe) of a register panel w
 // (row tid + NT*r of the block in w[r][.]) with implicit partial pivoting:
-// the pivot of each column is the unused row with the largest |re|+|im|
-// (lowest index on ties), as zgetf2 chooses.  Pivot rows get inP = tag.
+// the pivot of each column is the unused row with the largest |re|+|im|, to 17
+// bits; among rows that tie the last warp's, in a warp the lowest lane's.
+// Pivot rows get inP = tag.
 // One CTA barrier per step: every warp publishes its candidate (key,
 // reciprocal, updated row) into a slot double-buffered by step parity, so
 // after the barrier all threads read the winner's row directly.  The next

@@ -24,7 +24,8 @@
 // its panels.
 //
 // Measured on a B200, N = 221 with 28 channels open: a panel takes 95 thousand
-// cycles (a step's chain 3000, its FP64 work 500), the update of the other 189
+// cycles (a step's chain 3000, its FP64 work 500; 149 thousand from panel to
+// panel in a team, with the columns it needs and the cluster barrier), the update of the other 189
 // columns 126 thousand alone on the chip (94 thousand at the DMMA rate).  Nine
 // jobs of 160 slices 175 -> 86 ms.
 #pragma once
@@ -119,7 +120,8 @@ __device__ __forceinline__ void panel_sync(const PanelTeam &t) {
 
 // ------------------------------------------------------------ panel in registers
 // The pivot of column k of the basis, held by one warp in v (row lane + 32 r):
-// the scheme of reg_pivot; v becomes the multipliers, 0 in the pivot row.
+// the scheme of reg_pivot, to 16 bits of the magnitude; v becomes the
+// multipliers, 0 in the pivot row.
 template <int NRL>
 __device__ __forceinline__ void panel_pivot(double2 (&v)[NRL], unsigned free_rows, int k, int slot, double2 *scale,
                                             const PanelSmem &s) {

@@ -26,8 +26,8 @@
 // block is generated in exactly that order, element on element.
 //
 // Measured on a B200 against the global-memory kernel (8 x 1 x 2) it replaces
-// for these sizes: N = 69, N_z = 200, one energy 28.8 -> 15.6 ms, 512 energies
-// 80.5 -> 62.2 ms; N = 21, N_z = 60, one energy 1.91 -> 0.82 ms, 600 energies
+// for these sizes: N = 69, N_z = 200, one energy 28.6 -> 15.0 ms, 512 energies
+// 80.2 -> 61.2 ms; N = 21, N_z = 60, one energy 1.91 -> 0.82 ms, 600 energies
 // 6.2 -> 2.0 ms; N = 45, 400 energies 10.8 -> 5.5 ms.
 #pragma once
 #include "rgf_device.cuh"
@@ -133,7 +133,7 @@ __device__ __forceinline__ void reg_pivot(double2 (&v)[NRL], unsigned free_rows,
 // (tri_solve of 40 blocks of N = 69: error against 64 bits 0.84 of that of
 // scaled rows; with the 1 stored, 1.1 to 1.25 of it).  One barrier per step.  What bounds it is the chain from one pivot
 // to the next (about 1900 cycles a step at N = 69, of which the FP64 pipes are
-// busy for 500), so the warp that owns the next column brings that column up to
+// busy for 470), so the warp that owns the next column brings that column up to
 // date, publishes the next multipliers and goes straight to the next barrier;
 // the rest of its update follows behind that.
 template <int NRL, int PR, int CPW, int RPL, typename S>

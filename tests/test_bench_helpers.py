@@ -47,3 +47,13 @@ def test_reference_arm_loads_no_library_of_this_package():
     line = [l for l in out.stdout.splitlines() if l.startswith("NATIVE")][-1]
     assert line == "NATIVE False True", line
     assert '"impl": "reference"' in out.stdout
+
+
+@pytest.mark.parametrize("N,jobs,most_open,kernel,launches", [
+    (72, 512, 72, "k_register", 2), (73, 74, 73, "k_panel", 2), (160, 74, 160, "k_panel", 2), (161, 74, 160, "k_transmission<8,1,1>", 4),
+    (221, 74, 99, "k_panel", 4), (221, 74, 100, "k_transmission<8,1,1>", 4), (221, 18, 198, "k_panel", 4),
+    (256, 148, 20, "k_transmission<8,1,1>", 2), (256, 149, 20, "k_transmission<8,1,2>", 2),
+    (272, 500, 48, "k_panel", 4), (272, 500, 49, "k_transmission<16,2,1>", 4), (273, 1, 9, "k_transmission<16,2,1>", 2),
+    (513, 1, 9, "k_transmission<8,4,1>", 2)])
+def test_fp64_kernel_label(N, jobs, most_open, kernel, launches):
+    assert bench.fp64_kernel(N, jobs, 148, most_open) == (kernel, launches)
